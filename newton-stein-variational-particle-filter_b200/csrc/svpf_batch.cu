@@ -37,6 +37,7 @@ struct svpf_batch {
     std::vector<svpf_config_t> cfgs;
     std::vector<SVPFParams> prms;
     std::vector<uint8_t> tiles;
+    std::vector<uint8_t> fast;   // the filter's ticks go through the fast sums
     // device
     int* d_n = nullptr;
     long long* d_off = nullptr;
@@ -146,12 +147,14 @@ void drop_graph(svpf_batch* b) {
 }
 
 int upload_tiles(svpf_batch* b) {
+    std::vector<uint8_t> code(b->F);
     for (int f = 0; f < b->F; ++f) {
         const int t = tuned_batch_tile(b->ns[f]);
         b->tiles[f] = (uint8_t)(t >= kBatchTileLo && t <= kBatchTileHi ? t : default_batch_tile(b->ns[f]));
+        b->fast[f] = fast_tick(b->ns[f], b->cfgs[f]) ? 1 : 0;
+        code[f] = (uint8_t)(b->tiles[f] | (b->fast[f] ? kTileFast : 0));
     }
-    return cudaMemcpy(b->d_tile, b->tiles.data(), b->F, cudaMemcpyHostToDevice) == cudaSuccess ? SVPF_OK
-                                                                                              : SVPF_ERR_CUDA;
+    return cudaMemcpy(b->d_tile, code.data(), b->F, cudaMemcpyHostToDevice) == cudaSuccess ? SVPF_OK : SVPF_ERR_CUDA;
 }
 
 }  // namespace
@@ -163,6 +166,7 @@ svpf_batch_t* svpf_batch_create(int F, const int* ns, const svpf_config_t* cfgs,
     SVPF_TRACE();
     if (F < 1 || !ns || !cfgs || !prms) return nullptr;
     int n_max = 0, n_max1 = 0, n_max2 = 0, F1 = 0, heun = 0, prod = 1;
+    size_t smem1 = 0;
     for (int f = 0; f < F; ++f) {
         if (ns[f] < 1 || ns[f] > SVPF_MAX_PARTICLES || !config_loops_ok(cfgs[f])) return nullptr;
         n_max = std::max(n_max, ns[f]);
@@ -176,7 +180,9 @@ svpf_batch_t* svpf_batch_create(int F, const int* ns, const svpf_config_t* cfgs,
             ++F1;
         }
     }
-    if (F1 > 0 && tick_smem_bytes(n_max1, 1, heun != 0) > max_dyn_smem()) return nullptr;
+    for (int f = 0; f < F; ++f)
+        if (!cfgs[f].use_two_factor) smem1 = std::max(smem1, tick_smem_bytes_batch(ns[f], cfgs[f], heun != 0));
+    if (F1 > 0 && smem1 > max_dyn_smem()) return nullptr;
     if (F1 < F && tick_smem_bytes_2f(n_max2, 1) > max_dyn_smem()) return nullptr;
     svpf_batch* b = new svpf_batch();
     b->heun = heun;
@@ -193,6 +199,7 @@ svpf_batch_t* svpf_batch_create(int F, const int* ns, const svpf_config_t* cfgs,
     b->cfgs.assign(cfgs, cfgs + F);
     b->prms.assign(prms, prms + F);
     b->tiles.assign(F, 0);
+    b->fast.assign(F, 0);
     b->offs.resize(F);
     long long off = 0;
     for (int f = 0; f < F; ++f) {
@@ -239,7 +246,7 @@ svpf_batch_t* svpf_batch_create(int F, const int* ns, const svpf_config_t* cfgs,
          cudaMemset(b->d_lw, 0, b->total * sizeof(float)) == cudaSuccess;
     ok = ok && upload_tiles(b) == SVPF_OK;
     if (ok && b->F1 > 0) {
-        b->smem = tick_smem_bytes(n_max1, 1, heun != 0);
+        b->smem = smem1;
         b->grid = batch_grid(b->smem);
         ok = b->grid > 0;
     }
@@ -633,6 +640,7 @@ int svpf_batch_set_tile(svpf_batch_t* b, int f, int R, int S) {
     if (tile < 0) return SVPF_ERR_INVALID_ARG;
     if (cudaStreamSynchronize(b->stream) != cudaSuccess) return SVPF_ERR_CUDA;
     b->tiles[f] = (uint8_t)tile;
+    b->fast[f] = 0;   // a forced tile is the one that runs
     drop_graph(b);
     return cudaMemcpy(b->d_tile + f, &b->tiles[f], 1, cudaMemcpyHostToDevice) == cudaSuccess ? SVPF_OK
                                                                                           : SVPF_ERR_CUDA;

@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(kThreads, 2) batch_tick_kernel(const __grid_co
     __shared__ svpf_config_t cfg;
     __shared__ SVPFParams prm;
     __shared__ svpf_out_t out;
+    __shared__ FastSh fsh;
     __shared__ int s_next;
     const Team team{0, 1};
     for (;;) {
@@ -54,7 +55,10 @@ __global__ void __launch_bounds__(kThreads, 2) batch_tick_kernel(const __grid_co
         if (threadIdx.x == 0) pl.have_consts = 0;   // make_plan computes the per-tick constants
         if (!refuse_nonfinite(yt, ctl, out)) {   // a refused tick leaves the filter as it was
             const float ypr = readable_y_prev(yp);
-            switch (a.tile[f]) {
+            const int tile = a.tile[f];
+            if (tile & kTileFast) {
+                run_tick<2, 1, false, PROD, 0, true>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out, &fsh);
+            } else switch (tile) {
                 case 1: run_tick<1, 4, false, PROD>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
                 case 2: run_tick<1, 2, false, PROD>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
                 case 3: run_tick<1, 1, false, PROD>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;

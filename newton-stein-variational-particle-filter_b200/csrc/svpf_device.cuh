@@ -165,7 +165,7 @@ struct Plan {
     FactorPlan fac[2];     // two-factor: fast, slow
     float fmean[2];        // two-factor: factor means of the previous tick (guide)
     float gmean2[2];       // two-factor: EKF guide means
-    float red[4][kWarps];  // block reduction scratch
+    float red[5][kWarps];  // block reduction scratch
     float ksd_slot[kMaxCluster];
 };
 
@@ -319,7 +319,7 @@ __device__ __forceinline__ float warp_min(float v) {
     return v;
 }
 
-// Reduce up to four values (op per slot: 0 sum, 1 max, 2 min); result visible
+// Reduce up to five values (op per slot: 0 sum, 1 max, 2 min); result visible
 // to all threads.  Contains two __syncthreads.
 template <int K>
 __device__ __forceinline__ void block_reduce(float (&v)[K], const int (&op)[K], Plan& pl) {

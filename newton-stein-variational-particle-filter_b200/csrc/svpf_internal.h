@@ -27,6 +27,21 @@ inline bool is_production_tick(const svpf_config_t& c) {
     return c.use_newton && c.use_full_newton && !c.use_heun && !c.use_student_t_state;
 }
 
+// The fast sums (svpf_fast.cuh) take a filter's Stein iterations from this
+// many particles on.  592 production filters of one size, full budget, best
+// sweeps against fast sums per tick on B200: N = 192 251 / 389 us, 256 308 /
+// 420, 320 567 / 532, 384 644 / 541, 512 931 / 627; vanilla transport: 256
+// 296 / 386, 320 529 / 406.  The sweeps take 256 rows in one go, so their time
+// jumps just past that.
+constexpr int kFastMinN = 257;
+// Bit of a filter's tile byte: its ticks go through the fast sums; the tile is
+// the one its sweeps use when the particles do not fit them.
+constexpr int kTileFast = 0x80;
+SVPF_HD inline bool fast_tick(int n, const svpf_config_t& c) {
+    return n >= kFastMinN && !c.use_two_factor && !c.use_heun && !c.use_student_t_state &&
+           (!c.use_newton || c.use_full_newton);
+}
+
 struct SingleArgs {
     svpf_config_t cfg;
     SVPFParams prm;
@@ -109,6 +124,8 @@ struct InitArgs {
 // Dynamic shared-memory bytes of a tick kernel for n particles on C CTAs
 // (single-factor, and two-factor).
 size_t tick_smem_bytes(int n, int C, bool heun);
+// The batch kernel's for a filter: the larger of the sweeps' and the fast sums' layouts.
+size_t tick_smem_bytes_batch(int n, const svpf_config_t& c, bool heun);
 // The single-filter kernel's: the tick's layout plus the pre-drawn SVLD normals.
 size_t tick_smem_bytes_single(int n, int C, bool heun);
 size_t tick_smem_bytes_2f(int n, int C);

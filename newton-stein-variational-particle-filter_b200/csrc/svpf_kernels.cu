@@ -68,6 +68,11 @@ __global__ void philox_kernel(uint32_t k0, uint32_t k1, const uint32_t* ctr, uin
 // host side
 // ---------------------------------------------------------------------------
 size_t tick_smem_bytes(int n, int C, bool heun) { return (size_t)smem_floats(n, C, heun) * sizeof(float); }
+size_t tick_smem_bytes_batch(int n, const svpf_config_t& c, bool heun) {
+    const int sweeps = smem_floats(n, 1, heun);
+    const int fast = fast_tick(n, c) ? fast_smem_floats(n) : 0;
+    return (size_t)(fast > sweeps ? fast : sweeps) * sizeof(float);
+}
 size_t tick_smem_bytes_single(int n, int C, bool heun) {
     return (size_t)(smem_floats(n, C, heun) + pre_floats(n, C)) * sizeof(float);
 }
@@ -95,7 +100,7 @@ size_t max_dyn_smem() {
         int v = 0;
         if (cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
         const size_t static_bytes = sizeof(Plan) + sizeof(svpf_ctl_t) + sizeof(svpf_config_t) +
-                                    sizeof(SVPFParams) + sizeof(svpf_out_t) + 64;
+                                    sizeof(SVPFParams) + sizeof(svpf_out_t) + sizeof(FastSh) + 64;
         g_max_dyn_smem[dev] = (size_t)v > static_bytes ? (size_t)v - static_bytes : 0;
     }
     return g_max_dyn_smem[dev];

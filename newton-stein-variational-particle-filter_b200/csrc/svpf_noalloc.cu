@@ -89,7 +89,7 @@ __global__ void noalloc_setup_kernel(int F, const int* __restrict__ n, const lon
             tiles[f] = 0;   // no batch tile is 0: marks the filter as left out
             atomicAdd(&n_bad, 1);
         } else {
-            tiles[f] = (uint8_t)tile_for(nf);
+            tiles[f] = (uint8_t)(tile_for(nf) | (fast_tick(nf, c) ? kTileFast : 0));
             atomicAdd(&hist[bucket_of(nf)], 1);
         }
     }
@@ -151,7 +151,9 @@ int svpf_batch_tick_noalloc(int n_filters, const int* d_n, const long long* d_of
     if (!d_n || !d_off || !d_cfg || !d_params || !d_ctl || !d_h || !d_h_prev || !d_v || !d_log_w || !d_y_t ||
         !d_y_prev)
         return SVPF_ERR_INVALID_ARG;
-    const size_t smem = tick_smem_bytes(n_max, 1, any_heun != 0);
+    svpf_config_t any;   // the default configuration takes the fast sums
+    svpf_config_init(&any, 1, SVPF_DEFAULT_NU);
+    const size_t smem = tick_smem_bytes_batch(n_max, any, any_heun != 0);
     if (smem > max_dyn_smem()) return SVPF_ERR_INVALID_ARG;
     int err = SVPF_OK;
     int* scratch = scratch_for_current_device(&err);

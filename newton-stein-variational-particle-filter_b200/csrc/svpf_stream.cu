@@ -230,7 +230,9 @@ svpf_stream_t* svpf_stream_create(int max_instruments, size_t hbm_budget_bytes, 
         s->tiles.assign(C, 0);
         // shared memory sized for n_max; a model whose layout does not fit is
         // refused at admission
-        s->smem1 = tick_smem_bytes(n_max, 1, false);
+        svpf_config_t any;   // the default configuration takes the fast sums
+        svpf_config_init(&any, 1, SVPF_DEFAULT_NU);
+        s->smem1 = tick_smem_bytes_batch(n_max, any, false);
         s->smem2 = tick_smem_bytes_2f(n_max, 1);
         if (s->smem1 <= max_dyn_smem()) s->grid1 = batch_grid(s->smem1);
         if (s->smem2 <= max_dyn_smem()) s->grid2 = batch_grid_2f(s->smem2);
@@ -303,7 +305,8 @@ int svpf_stream_admit(svpf_stream_t* s, int n, const svpf_config_t* cfg, const S
     s->used_floats += (size_t)L;
     {
         const int t = tuned_batch_tile(n);
-        s->tiles[slot] = (uint8_t)(t >= kBatchTileLo && t <= kBatchTileHi ? t : default_batch_tile(n));
+        s->tiles[slot] = (uint8_t)((t >= kBatchTileLo && t <= kBatchTileHi ? t : default_batch_tile(n)) |
+                                   (fast_tick(n, *cfg) ? kTileFast : 0));
     }
     // control record as svpf_initialize leaves it (svpf_optimized_graph.cu:349-451)
     svpf_config_t c = *cfg;

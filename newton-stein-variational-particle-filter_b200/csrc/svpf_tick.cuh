@@ -6,6 +6,7 @@
 #pragma once
 
 #include "svpf_device.cuh"
+#include "svpf_fast.cuh"
 
 namespace svpf {
 
@@ -85,6 +86,222 @@ __device__ __forceinline__ void flag_y_prev(float y_prev, svpf_ctl_t& ctl) {
     if (threadIdx.x == 0 && !isfinite(y_prev) && ctl.status == SVPF_OK) ctl.status = SVPF_ERR_NONFINITE;
 }
 
+// Prior mean of a particle at h (svpf_opt_kernels.cu:384-392).
+__device__ __forceinline__ float prior_mean(float h, const Plan& pl, const SVPFParams& prm, float y_prev) {
+    const float lev = prm.gamma * y_prev;
+    return pl.mu_eff + prm.rho * (h - pl.mu_eff) + (lev != 0.0f ? lev / (expf(h * 0.5f) + 1e-8f) : 0.0f);
+}
+
+// Workspace of the fast tick (one CTA): particle-order and slot-order arrays
+// of n floats, the slots' particles, the tables (svpf_fast.cuh).
+struct FastWork {
+    float* a;                 // positions in particle order; g by slot once they are binned
+    float* b;                 // positions by slot
+    float* c;                 // curvature by slot; then the next positions in particle order
+    unsigned short* pidx;     // particle of a slot
+    FastTab tab;
+    Sources src;              // the prior means
+    int sft;                  // fine bins of a mixture panel, log2
+};
+
+// Floats of dynamic shared memory of a fast tick.
+__host__ __device__ inline int fast_smem_floats(int n) {
+    const int np = round_up(n, 64);
+    return 3 * np + np / 2 + fast_table_floats(true);
+}
+
+// The scaled prior means (w.c) as points, once per tick, in panels of 0.75
+// scaled units, or of 1.5 where that many do not fit.  False: they do not fit,
+// or one fine bin is too wide for the mixture.
+__device__ inline bool fast_sources(FastWork& w, const Plan& pl, int n, FastSh& sh) {
+    const float unit = pl.bw * pl.prior_scale;   // scaled units per bandwidth
+    w.sft = 3;
+    while (w.sft > 0 && kFineW * unit * (float)(1 << w.sft) > kMixPanelMax) --w.sft;
+    if (!(kFineW * unit * (float)(1 << w.sft) <= kMixPanelMax)) return false;
+    const FastTab& t = w.tab;
+    for (int wide = 0; wide < 2; ++wide) {
+        w.src.up = wide ? 0.5f : 1.0f;
+        w.src.near = wide ? 0 : 3;
+        w.src.far2 = wide ? 5.0625f : 20.25f;
+        fast_bin(w.c, n, kFineScale * w.src.up, w.b, w.pidx, t, sh);
+        const Panels p = fast_panels(3, t.src_pt, t.comp, kFineBins / kFine, kMaxSrc, true, t, sh);
+        if (sh.over) {
+            __syncthreads();   // everyone has read it
+            continue;
+        }
+        w.src.ns = p.m;
+        if (threadIdx.x == 0) t.src_pt[kFineBins / kFine] = (unsigned short)p.m;
+        const int pad = min(round_up(p.m, 4), kMaxSrc);
+        fast_points(w.b, w.src.up, t, p, t.src_x, pad, kMuPad);
+        auto none = [](int) { return 0.0f; };
+        fast_weights<false, false, false>(w.b, w.src.up, t, p, t.src_w, nullptr, nullptr, none, none);
+        for (int i = p.m + threadIdx.x; i < pad; i += kThreads) t.src_w[i] = 0.0f;
+        __syncthreads();
+        return true;
+    }
+    return false;
+}
+
+// One Stein iteration of a filter on one CTA through the fast sums
+// (svpf_fast.cuh): gradient pass (svpf_opt_kernels.cu:354-521), vanilla or
+// full-Newton transport (:527-1103) as grad_pass and transport_pass take it.
+// Positions: w.a before, w.c after (w.a untouched when it returns false: the
+// particles do not fit the tables).  ksd: this thread's KSD terms.
+template <bool PROD>
+__device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_config_t& cfg, const SVPFParams& prm,
+                               const FilterIO& io, const Noise& nz, int kn, float beta, float bf, bool last,
+                               FastSh& sh, float& ksd) {
+    const int tid = threadIdx.x, n = io.n;
+    const FastTab& t = w.tab;
+    fast_bin(w.a, n, kFineScale, w.b, w.pidx, t, sh);
+    const Panels p = fast_panels(3, t.pt, t.comp, kMaxComp, kMaxPts, false, t, sh);
+    // the mixture's panels: the same ones unless they are too many sigma wide
+    const Panels q = w.sft == 3 ? p : fast_panels(w.sft, t.mpt, t.mcomp, kMixComp, kMixPts, false, t, sh);
+    if (sh.over) return false;
+    fast_points(w.b, 1.0f, t, q, t.pts, q.m, kHPad);
+    __syncthreads();
+    auto scaled = [&](float x) { return (fmaf(x, pl.bw, pl.center) - pl.mu_center) * pl.prior_scale; };
+    auto mean = [&](int k) { return (prior_mean(io.h[k], pl, prm, pl.y_prev) - pl.mu_center) * pl.prior_scale; };
+    fast_mixture_points(t, sh, q.m, w.src, n, scaled, mean);
+    __syncthreads();
+    fast_mixture_panels(t, q, pl.bw * pl.prior_scale);
+    __syncthreads();
+    const int kind = PROD ? 2 : pl.transport;
+    const float inv_s2 = 1.0f / (pl.sz_eff * pl.sz_eff);
+    const float nu = cfg.nu;
+    const float y2 = pl.y_t * pl.y_t;
+    for (int base = 0; base < n; base += kThreads) {
+        const int s = base + tid;
+        const bool on = s < n;
+        const float x = w.b[min(s, n - 1)];
+        const int b = fine_bin(x) >> q.sft;
+        const int j0 = t.fstart[b << q.sft];
+        const bool comp = q.interpolated(b, t.fstart[(b + 1) << q.sft] - j0);
+        const int at = q.pt[b];
+        float den, num;
+        if (comp) {
+            float T[kP];
+            cheb(q.local(x, b), T);
+            den = cheb_dot(T, t.pts + kMixPts + at);
+            num = cheb_dot(T, t.pts + 2 * kMixPts + at);
+        } else {
+            const int r = at + (min(s, n - 1) - j0);
+            den = t.pts[kMixPts + r];
+            num = t.pts[2 * kMixPts + r];
+        }
+        unsigned todo = __ballot_sync(0xffffffffu, on && comp && t.bad[at / kP]);
+        while (todo) {
+            const int src = __ffs(todo) - 1;
+            todo &= todo - 1u;
+            float d_, n_;
+            mixture_warp(__shfl_sync(0xffffffffu, scaled(x), src), t, w.src, n, mean, d_, n_);
+            if ((tid & 31) == src) {
+                den = d_;
+                num = n_;
+            }
+        }
+        if (!on) continue;
+        // likelihood, combination and curvature as in grad_pass
+        const float h = fmaf(x, pl.bw, pl.center);
+        const float gp = -(num / pl.prior_scale) * inv_s2 / den;
+        const float vol = expf(fminf(h, 20.0f));
+        const float A = y2 / (vol + 1e-8f) / nu;
+        const float opA = 1.0f + A;
+        float glik;
+        if (cfg.use_exact_gradient) glik = -0.5f + 0.5f * (nu + 1.0f) * A / opA - cfg.lik_offset;
+        else glik = (logf(y2 + 1e-10f) - h + cfg.lik_offset) / 1.4f;
+        const float eb = pl.fan ? 1.0f : beta;
+        w.a[s] = clampf(gp + eb * glik, -10.0f, 10.0f);
+        if (kind == 2) {
+            const float hl = -0.5f * (nu + 1.0f) * A / (opA * opA);
+            w.c[s] = clampf(-(hl - inv_s2), 0.1f, 100.0f);
+        }
+        if (last)
+            io.lw[w.pidx[s]] = pl.fan ? 0.0f
+                                      : pl.stc - 0.5f * h - (nu + 1.0f) * 0.5f * log1pf(fmaxf(A, -0.999f));
+    }
+    __syncthreads();
+    const int m = p.m, m_pad = round_up(m, 32);
+    fast_points(w.b, 1.0f, t, p, t.pts, m_pad, kHPad);
+    for (int i = m + tid; i < m_pad; i += kThreads)
+        t.pts[kMaxPts + i] = t.pts[2 * kMaxPts + i] = t.pts[3 * kMaxPts + i] = 0.0f;
+    auto gv = [&](int j) { return w.a[j]; };
+    auto cv = [&](int j) { return w.c[j]; };
+    if (kind == 2)
+        fast_weights<true, true, true>(w.b, 1.0f, t, p, t.pts + kMaxPts, t.pts + 2 * kMaxPts, t.pts + 3 * kMaxPts, gv, cv);
+    else
+        fast_weights<true, false, false>(w.b, 1.0f, t, p, t.pts + kMaxPts, t.pts + 2 * kMaxPts, nullptr, gv, cv);
+    __syncthreads();
+    if (kind == 2) {
+        if (last) fast_point_sums<true, true>(t, m, m_pad);
+        else fast_point_sums<true, false>(t, m, m_pad);
+    } else {
+        if (last) fast_point_sums<false, true>(t, m, m_pad);
+        else fast_point_sums<false, false>(t, m, m_pad);
+    }
+    __syncthreads();
+    if (kind == 2) {
+        fast_coefficients(t, p.nc, 4, last ? 7 : 5);
+    } else {
+        fast_coefficients(t, p.nc, 4, 2);
+        if (last) fast_coefficients(t, p.nc, 9, 2);
+    }
+    __syncthreads();
+    const float sign = cfg.stein_repulsive_sign == 1 ? 1.0f : -1.0f;
+    const float inv_bw = pl.inv_bw, inv_bw2 = pl.inv_bw2, inv_n = 1.0f / (float)n;
+    const float es = pl.eps_step * bf, rr = cfg.rmsprop_rho;
+    ksd = 0.0f;
+    for (int s = tid; s < n; s += kThreads) {
+        const float x = w.b[s];
+        const int i = w.pidx[s];
+        const float v0 = io.v[i];
+        const int b = fine_bin(x) / kFine;
+        const int j0 = t.fstart[kFine * b];
+        float sum[7] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        const float* row = t.pts + 4 * kMaxPts + p.pt[b];
+        if (p.interpolated(b, t.fstart[kFine * (b + 1)] - j0)) {
+            float T[kP];
+            cheb(p.local(x, b), T);
+            sum[0] = cheb_dot(T, row);
+            sum[1] = cheb_dot(T, row + kMaxPts);
+            if (kind == 2) {
+                sum[2] = cheb_dot(T, row + 2 * kMaxPts);
+                sum[3] = cheb_dot(T, row + 3 * kMaxPts);
+                sum[4] = cheb_dot(T, row + 4 * kMaxPts);
+            }
+            if (last) {
+                sum[5] = cheb_dot(T, row + 5 * kMaxPts);
+                sum[6] = cheb_dot(T, row + 6 * kMaxPts);
+            }
+        } else {
+            row += s - j0;
+#pragma unroll
+            for (int k = 0; k < 7; ++k)
+                if (k < 2 || (k < 5 ? kind == 2 : last)) sum[k] = row[k * kMaxPts];
+        }
+        float phi = (sum[0] + sign * 2.0f * inv_bw * sum[1]) * inv_n;
+        if (kind == 2) {
+            const float nk = sum[4] + 2.0f * fast_window(x, w.b, t, p);
+            float H = (sum[3] + 2.0f * inv_bw2 * nk) / fmaxf(sum[2], 1e-6f);
+            H = clampf(H, 0.1f, 100.0f);
+            phi = phi * (1.0f / H) * 0.7f;
+        }
+        if (last) {
+            const float si = w.a[s];
+            ksd += si * sum[0] + 2.0f * inv_bw * (si * sum[1] - sum[5]) + 2.0f * inv_bw2 * sum[6];
+        }
+        const float vn = rr * v0 + (1.0f - rr) * phi * phi;
+        io.v[i] = vn;
+        const float drift = es * phi * rsqrtf(vn + cfg.rmsprop_eps);
+        float diff = 0.0f;
+        if (pl.temp > 1e-6f) diff = sqrtf(2.0f * es * pl.temp) * nz.normal(i, kn);
+        const float h_new = clamp_h(fmaf(x, pl.bw, pl.center) + drift + diff);
+        w.c[i] = (h_new - pl.center) * inv_bw;
+    }
+    __syncthreads();
+    return true;
+}
+
 // The tick.  cfg/prm/ctl are shared-memory copies owned by the caller; only
 // thread 0 of rank 0 mutates ctl after make_plan.  Returns on every member; the
 // caller stores ctl/out from rank 0 thread 0.  SCAN: the mixture's row
@@ -93,27 +310,43 @@ __device__ __forceinline__ void flag_y_prev(float y_prev, svpf_ctl_t& ctl) {
 // caller guarantees full-Newton transport, Gaussian state noise and no Heun
 // step (the production configuration), so only those code paths are compiled
 // and the kernel body stays small (instruction fetch bounds the latency kernel).
-template <int R, int S, bool SCAN = false, bool PROD = false, int U = 0>
+// FAST: the Stein iterations go through the fast sums (one CTA, Gaussian state
+// noise, vanilla or full-Newton transport, no Heun step, dynamic shared memory
+// of fast_smem_floats); a tick whose particles do not fit them finishes with
+// the <R, S> sweeps.
+template <int R, int S, bool SCAN = false, bool PROD = false, int U = 0, bool FAST = false>
 __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_ctl_t& ctl, float y_t,
                          float y_prev, const FilterIO& io, const Noise& nz, const Smem& sm, Plan& pl,
-                         const Team& team, svpf_out_t& out) {
+                         const Team& team, svpf_out_t& out, FastSh* fsh = nullptr) {
     const int tid = threadIdx.x;
     const int n = sm.n;
+    FastWork fw;
+    if constexpr (FAST) {
+        fw.a = sm.h[0];
+        fw.b = sm.h[1];
+        fw.c = sm.g;
+        fw.pidx = reinterpret_cast<unsigned short*>(sm.c);
+        fw.tab = carve_fast(sm.c + sm.np / 2, true);
+        fast_load_tables(fw.tab);
+    }
     if (tid == 0) {
         pl.flag = 0;
         make_plan(cfg, prm, ctl, y_t, y_prev, pl);
         if (cfg.use_heun) pl.transport = (cfg.use_newton && cfg.use_full_newton) ? 2 : 0;
     }
     // pads: particle columns [n, np) and prior slots [n, m_len)
-    for (int i = n + tid; i < sm.np; i += kThreads) {
-        sm.h[0][i] = kHPad; sm.h[1][i] = kHPad; sm.g[i] = 0.0f; sm.c[i] = 0.0f;
-    }
-    for (int i = n + tid; i < sm.m_len; i += kThreads) sm.mu[i] = kMuPad;
+    auto pads = [&]() {
+        for (int i = n + tid; i < sm.np; i += kThreads) {
+            sm.h[0][i] = kHPad; sm.h[1][i] = kHPad; sm.g[i] = 0.0f; sm.c[i] = 0.0f;
+        }
+        for (int i = n + tid; i < sm.m_len; i += kThreads) sm.mu[i] = kMuPad;
+    };
+    if constexpr (!FAST) pads();
     __syncthreads();
 
     // ---- predict (svpf_opt_kernels.cu:125-276), guide (:282-327), prior means
     //      (:384-392); every team member does all N rows, no exchange needed.
-    float st[4] = {0.0f, 0.0f, 1e10f, -1e10f};
+    float st[FAST ? 5 : 4] = {0.0f, 0.0f, 1e10f, -1e10f};
     {
         const float hbar = ctl.h_mean_prev;
         const bool mim = cfg.use_mim || cfg.use_guided;
@@ -161,14 +394,23 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
                 hp = cfg.use_guide_preserving ? clamp_h(nm_pres + (hp - hbar)) : clamp_h(hp + gsn * (gmean - hp));
             }
             sm.h[0][i] = hp;
-            sm.mu[i] = pl.mu_eff + prm.rho * (hi - pl.mu_eff) + prm.gamma * y_prev / (expf(hi * 0.5f) + 1e-8f);
+            if constexpr (FAST) {
+                const float mk = prior_mean(hi, pl, prm, y_prev);
+                sm.g[i] = mk;
+                st[4] += mk;
+            } else {
+                sm.mu[i] = pl.mu_eff + prm.rho * (hi - pl.mu_eff) + prm.gamma * y_prev / (expf(hi * 0.5f) + 1e-8f);
+            }
             st[0] += hp;
             st[1] += hp * hp;
             st[2] = fminf(st[2], hp);
             st[3] = fmaxf(st[3], hp);
         }
     }
-    {
+    if constexpr (FAST) {
+        const int op[5] = {0, 0, 2, 1, 0};
+        block_reduce<5>(st, op, pl);
+    } else {
         const int op[4] = {0, 0, 2, 1};
         block_reduce<4>(st, op, pl);
     }
@@ -197,11 +439,12 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
         pl.inv_bw = 1.0f / bw;
         pl.inv_bw2 = 1.0f / (bw * bw);
         pl.center = mean;
-        pl.mu_center = pl.mu_eff;
+        if constexpr (FAST) pl.mu_center = st[4] * inv_n;   // the panels of the prior means are centred on them
+        else pl.mu_center = pl.mu_eff;
         pl.prior_scale = sqrtf(kLog2e * 0.5f / (pl.sz_eff * pl.sz_eff));
     }
     // ---- sort prior means once per tick (used for the per-row maximum)
-    if constexpr (!SCAN) bitonic_sort(sm.mu, sm.p2);
+    if constexpr (!SCAN && !FAST) bitonic_sort(sm.mu, sm.p2);
     else __syncthreads();   // plan scalars of thread 0 visible to all
     // ---- Stein-loop coordinates: positions (h - center) / bw, Gaussian prior
     //      means (mu - mu_center) * prior_scale (order preserving)
@@ -209,11 +452,14 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
     if (pl.budget > 0) {
         for (int i = tid; i < n; i += kThreads) {
             sm.h[0][i] = (sm.h[0][i] - pl.center) * pl.inv_bw;
-            if (!student) sm.mu[i] = (sm.mu[i] - pl.mu_center) * pl.prior_scale;
+            if constexpr (FAST) sm.g[i] = (sm.g[i] - pl.mu_center) * pl.prior_scale;
+            else if (!student) sm.mu[i] = (sm.mu[i] - pl.mu_center) * pl.prior_scale;
         }
     }
-    // ---- own rows' RMSProp state
-    for (int li = tid; li < sm.row1 - sm.row0; li += kThreads) sm.v[li] = io.v[sm.row0 + li];
+    // ---- own rows' RMSProp state (the fast iterations keep it in global memory)
+    if constexpr (!FAST) {
+        for (int li = tid; li < sm.row1 - sm.row0; li += kThreads) sm.v[li] = io.v[sm.row0 + li];
+    }
     // ---- SVLD normals of own rows for the first Stein iterations, drawn in
     //      parallel (same draws, in the same slots, as the per-row epilogue takes)
     if (sm.pre != nullptr && pl.temp > 1e-6f && (PROD || !cfg.use_heun)) {
@@ -230,7 +476,41 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
     int cur = 0;
     int kn = pl.kn_pred;
     const int budget = pl.budget;
-    for (int it = 0; it < budget; ++it) {
+    int it0 = 0;
+    bool direct = !FAST;
+    if constexpr (FAST) {
+        if (budget > 0) {
+            bool fits = fast_sources(fw, pl, n, *fsh);
+            while (fits && it0 < budget) {
+                const float beta = pl.beta[stage_of(pl, it0)];
+                float kt;
+                fits = fast_iteration<PROD>(fw, pl, cfg, prm, io, nz, kn, beta, sqrtf(beta), it0 == budget - 1, *fsh, kt);
+                if (!fits) break;
+                if (it0 == budget - 1) ksd_publish(kt, pl, team);
+                float* x = fw.c;
+                fw.c = fw.a;
+                fw.a = x;
+                if (pl.temp > 1e-6f) ++kn;
+                ++it0;
+            }
+            if (!fits) {
+                // the sweeps take over: positions, prior means (sorted) and moments where they expect them
+                __syncthreads();
+                direct = true;
+                if (fw.a != sm.h[0])
+                    for (int i = tid; i < n; i += kThreads) sm.h[0][i] = fw.a[i];
+                __syncthreads();
+                pads();
+                for (int i = tid; i < n; i += kThreads) {
+                    sm.mu[i] = (prior_mean(io.h[i], pl, prm, y_prev) - pl.mu_center) * pl.prior_scale;
+                    sm.v[i] = io.v[i];
+                }
+                __syncthreads();
+                bitonic_sort(sm.mu, sm.p2);
+            }
+        }
+    }
+    for (int it = it0; it < budget; ++it) {
         const int ai = stage_of(pl, it);
         const float beta = pl.beta[ai];
         const float bf = sqrtf(beta);
@@ -297,7 +577,9 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
     }
 
     // own rows' RMSProp state back to global memory
-    for (int li = tid; li < sm.row1 - sm.row0; li += kThreads) io.v[sm.row0 + li] = sm.v[li];
+    if (direct) {
+        for (int li = tid; li < sm.row1 - sm.row0; li += kThreads) io.v[sm.row0 + li] = sm.v[li];
+    }
     if (team.rank != 0) return;
 
     if (tid == 0) {
@@ -312,6 +594,8 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
 
     // ---- back to log-volatility coordinates
     float* hf = sm.h[cur];
+    if constexpr (FAST)
+        if (!direct) hf = fw.a;
     if (budget > 0) {
         for (int i = tid; i < n; i += kThreads) hf[i] = fmaf(hf[i], pl.bw, pl.center);
         __syncthreads();

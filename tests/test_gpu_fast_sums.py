@@ -1,0 +1,96 @@
+"""The batch tick's fast sums (csrc/svpf_fast.cuh) against the FP64 oracle.
+
+A filter of 257 particles or more that has no forced tile takes its Stein
+iterations through interpolated panels instead of the sweeps over all pairs.
+One tick from made states, at sizes around the tiles' and bins' edges, where
+that path branches: a smooth cloud, one point (a single panel, equal
+particles), two clusters many sigma apart (mixture sums that do not
+interpolate), far outliers and particles at the position clamp (the shared
+edge panels), a shock that moves the particles away from the prior means (far
+points), and a spread that does not fit the tables (the sweeps finish the
+tick).  Tolerance as in the randomised runs: 1e-4 relative (floor 1; KSD
+1e-3), or four times what the oracle's own FP32 mirror deviates on the same
+state and on that state moved by two FP32 ulps.
+"""
+import concurrent.futures as cf
+import os
+
+import numpy as np
+import pytest
+
+import tape
+from test_gpu_batch_parity import _twin
+from test_oracle import TOL, rel_err
+
+pytestmark = pytest.mark.gpu
+
+STATES = ["cloud", "point", "clusters", "outliers", "clamped", "shock", "spread"]
+SIZES = [257, 300, 512, 777, 1025, 2049, 4096]
+
+
+def _state(kind, n, rng, mu):
+    if kind == "point":
+        h = np.full(n, mu)
+    elif kind == "clusters":
+        h = np.where(np.arange(n) % 3 == 0, mu + 2.0, mu - 1.0) + 0.02 * rng.standard_normal(n)
+    elif kind == "spread":
+        h = rng.uniform(-15.0, 5.0, n)
+    else:
+        h = mu + (0.1 if kind == "shock" else 0.5) * rng.standard_normal(n)
+        if kind == "outliers":
+            h[:: 23] = rng.uniform(-14.0, 4.5, len(h[:: 23]))
+        if kind == "clamped":
+            h[:: 3] = -15.0
+    return np.clip(h, -15.0, 5.0).astype(np.float32)
+
+
+@pytest.mark.parametrize("newton", [1, 0])
+@pytest.mark.parametrize("sigma", [0.05, 0.3])
+def test_fast_sums_match_oracle(pkg, oracle_mod, newton, sigma):
+    ns = [n for n in SIZES for _ in STATES] + [8192]
+    kinds = STATES * len(SIZES) + ["spread"]
+    F, n_max = len(ns), max(ns)
+    cfg = pkg.production_config(8.0, 5)
+    cfg.update(use_newton=newton, use_full_newton=newton, stein_min_steps=4, stein_max_steps=5)
+    params = [(0.95, sigma, -1.0, -0.2 if f % 2 else 0.0) for f in range(F)]
+    b = pkg.Batch(ns, [cfg] * F, [pkg.Params(*p) for p in params])
+    b.initialize(seed=3)
+    rng = np.random.default_rng(17)
+    y = np.empty(F, np.float32)
+    for f in range(F):
+        ctl = b.get_state(f)[0]
+        ctl.timestep, ctl.ksd_prev, ctl.ksd_last, ctl.vol_prev = 12, 0.6, 0.6, 0.6
+        ctl.guide_initialized, ctl.h_mean_prev, ctl.bw_sq = 1, -1.0, 0.04
+        ctl.return_ema, ctl.return_var = 0.5, 0.3
+        h = _state(kinds[f], ns[f], rng, -1.0)
+        v = rng.uniform(0.05, 0.5, ns[f]).astype(np.float32)
+        b.set_state(f, ctl, h, (h - 0.1).astype(np.float32), v, np.zeros(ns[f], np.float32))
+        y[f] = 25.0 if kinds[f] == "shock" else 0.4 + 0.05 * (f % 7)
+    nrm, uni = tape.tape(5, 0, n_max, 16, 2)
+    b.set_noise_tape(nrm, uni)
+    yp = np.full(F, 0.3, np.float32)
+    twins = [_twin(oracle_mod, b, f, cfg, params[f]) for f in range(F)]
+    mirrors = []
+    for nudge in (0.0, 2.0 ** -22, -(2.0 ** -22)):
+        m = [_twin(oracle_mod, b, f, cfg, params[f], 1) for f in range(F)]
+        for o in m:
+            o.h = o.h * (1.0 + nudge)
+        mirrors.append(m)
+    ll, vol, hm = b.step(y, yp)
+    ctl = b.ctl()
+    with cf.ThreadPoolExecutor(max_workers=min(16, os.cpu_count() or 1)) as pool:
+        def step(m):
+            return list(pool.map(lambda f: m[f].step(y[f], yp[f], nrm[:, :ns[f]], uni[:, :ns[f]]), range(F)))
+        want, around = step(twins), [step(m) for m in mirrors]
+    for f in range(F):
+        tag = (kinds[f], ns[f])
+        assert ctl[f].status == 0 and ctl[f].stein_steps_used == want[f].steps_used, tag
+        dev = max(rel_err(m[f].h, twins[f].h) for m in mirrors)
+        got = b.get_particles(f)
+        assert rel_err(got, twins[f].h) < max(TOL, 4 * dev), (tag, rel_err(got, twins[f].h), dev)
+        for name, value, base in (("loglik", ll[f], TOL), ("vol", vol[f], TOL), ("h_mean", hm[f], TOL),
+                                  ("ksd", ctl[f].ksd_last, 1e-3)):
+            w = getattr(want[f], name)
+            dev = max(abs(getattr(a[f], name) - w) for a in around) / max(1.0, abs(w))
+            assert abs(value - w) < max(base, 4 * dev) * max(1.0, abs(w)), (tag, name, value, w, dev)
+    b.close()
