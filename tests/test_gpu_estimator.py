@@ -177,3 +177,24 @@ def test_invalid_sizes_are_rejected(pkg):
         pkg.Estimator(1, 63, 2, 0.1, T_max=10)
     with pytest.raises(RuntimeError):
         pkg.Estimator(1, 64, 2, 0.1, T_max=0)
+
+
+@pytest.mark.parametrize("n, steps", [(2, 1), (30, 0), (64, 2), (98, 3), (256, 1), (258, 2)])
+def test_records_give_the_bits_of_the_checkpointed_path(pkg, n, steps):
+    """The backward from run records and the one that recomputes checkpoint
+    segments (an engine whose records would not fit) agree bit for bit, at
+    particle counts around the CTA sizes and the columns read at a time."""
+    P, T = 3, 9
+    rng = np.random.default_rng(n)
+    th = np.stack([rng.uniform(-4.0, -3.0, P), rng.uniform(0.85, 0.97, P), rng.uniform(0.1, 0.3, P),
+                   np.full(P, 8.0)], 1).astype(np.float32)
+    y = (0.2 * rng.standard_normal((P, T))).astype(np.float32)
+    out = []
+    # T_max sizes the records: 4 GiB of them are refused
+    for t_max in (T, 1 + (4 << 30) // (P * 4 * (4 + max(steps, 1)) * ((n + 63) // 64 * 64))):
+        e = pkg.Estimator(P, n, steps, 0.15, T_max=t_max, checkpoint_every=4, truncate_every=5)
+        ll, vol, _ = e.forward(th, y, seed=2)
+        out.append((ll, vol, e.backward()))
+        e.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
