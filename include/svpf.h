@@ -431,8 +431,8 @@ int svpf_batch_tile_of(const svpf_batch_t* b, int n, int* rows_per_thread, int* 
  * one: (rows_per_thread, col_split) must be a compiled batch tile, (1,4)
  * (1,2) (1,1) (2,1) (4,1); SVPF_ERR_INVALID_ARG otherwise.  Forcing a tile
  * waits for the batch's stream and drops its captured graph.  A filter large
- * enough for the fast sums (more than 256 particles, vanilla or full-Newton
- * transport, Gaussian state noise, no Heun step) sweeps over its pairs with a
+ * enough for the fast sums (more than 256 particles; two-factor, or vanilla or
+ * full-Newton transport, Gaussian state noise and no Heun step) sweeps over its pairs with a
  * tile only when the tile is forced, or when its particles do not fit the
  * sums' tables. */
 int svpf_batch_tile_of_filter(const svpf_batch_t* b, int filter, int* rows_per_thread, int* col_split);

@@ -151,7 +151,9 @@ int upload_tiles(svpf_batch* b) {
     for (int f = 0; f < b->F; ++f) {
         const int t = tuned_batch_tile(b->ns[f]);
         b->tiles[f] = (uint8_t)(t >= kBatchTileLo && t <= kBatchTileHi ? t : default_batch_tile(b->ns[f]));
-        b->fast[f] = fast_tick(b->ns[f], b->cfgs[f]) ? 1 : 0;
+        // (a two-factor filter's tables may not fit where its sweeps do)
+        b->fast[f] = fast_tick(b->ns[f], b->cfgs[f]) &&
+                     (!b->tf[f] || tick_smem_bytes_2f_fast(b->ns[f]) <= max_dyn_smem());
         code[f] = (uint8_t)(b->tiles[f] | (b->fast[f] ? kTileFast : 0));
     }
     return cudaMemcpy(b->d_tile, code.data(), b->F, cudaMemcpyHostToDevice) == cudaSuccess ? SVPF_OK : SVPF_ERR_CUDA;
@@ -252,6 +254,8 @@ svpf_batch_t* svpf_batch_create(int F, const int* ns, const svpf_config_t* cfgs,
     }
     if (ok && b->F2 > 0) {
         b->smem2 = tick_smem_bytes_2f(n_max2, 1);
+        for (int f = 0; f < F; ++f)
+            if (b->tf[f] && b->fast[f]) b->smem2 = std::max(b->smem2, tick_smem_bytes_2f_fast(ns[f]));
         b->grid2 = batch_grid_2f(b->smem2);
         ok = b->grid2 > 0;
     }

@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(kThreads, 2) batch_tick_2f_kernel(const __grid
     __shared__ svpf_config_t cfg;
     __shared__ SVPFParams prm;
     __shared__ svpf_out_t out;
+    __shared__ FastSh fsh;
     __shared__ int s_next;
     const Team team{0, 1};
     for (;;) {
@@ -97,7 +98,9 @@ __global__ void __launch_bounds__(kThreads, 2) batch_tick_2f_kernel(const __grid
         __syncthreads();
         const int n = a.n[f];
         const long long off = a.off[f];
-        const Smem2 sm = carve_2f(smem, n, 1, 0);
+        const int tile = a.tile[f];
+        FastWork2 fw;
+        const Smem2 sm = tile & kTileFast ? carve_2f_fast(smem, n, fw) : carve_2f(smem, n, 1, 0);
         const FilterIO io{a.h + off, a.hp + off, a.v + off, a.lw + off, n};
         const Noise nz{philox_key(a.seed, f), (uint32_t)ctl.timestep, a.tape_n, a.tape_u,
                        a.slots_n, a.slots_u, a.tape_stride, &pl.flag};
@@ -106,7 +109,9 @@ __global__ void __launch_bounds__(kThreads, 2) batch_tick_2f_kernel(const __grid
         const float yp = a.req_y ? ctl.y_prev : a.y_prev[f];
         if (!refuse_nonfinite(yt, ctl, out)) {   // a refused tick leaves the filter as it was
             const float ypr = readable_y_prev(yp);
-            switch (a.tile[f]) {
+            if (tile & kTileFast) {
+                run_tick_2f<1, 1, true>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out, &fw, &fsh);
+            } else switch (tile) {
                 case 1: run_tick_2f<1, 4>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
                 case 2: run_tick_2f<1, 2>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
                 case 3: run_tick_2f<1, 1>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;

@@ -44,7 +44,9 @@
 // against 4.7 M with the sweeps, one of N = 512 55 k against 100 k.  The batch
 // tick of 4096 filters (N 256 to 4096) went from 83.6 to 4.7 ms, its first
 // tick from 83 to 13 ms, 300 filters of 100 to 1500 particles from 4.0 to
-// 0.52 ms.
+// 0.52 ms.  The two-factor tick's transports (no mixture, no Hessian) take the
+// same way: a request round of 200 instruments of 256 to 2048 particles went
+// from 7.5 to 2.9 ms, bound by the ticks of N = 2048.
 #pragma once
 
 #include "svpf_device.cuh"
@@ -65,6 +67,7 @@ constexpr int kMixPts = 1408;            // points the mixture is summed at
 constexpr int kMixComp = kMixPts / kP;
 constexpr int kMaxSrc = 1280;            // points standing for the prior means
 constexpr int kPtRows = 11;              // arrays of kMaxPts floats
+constexpr int kMaxPts2f = 1120;          // two factors: 5 arrays of up to this many
 constexpr float kKink = 0.57735026918962576f;   // 3 u^2 = 1
 // Widest panel in the mixture's scaled units: at half-width 0.75 the Gaussian
 // sums interpolate to 6e-9 with kP points (2e-7 at half-width 1).
@@ -164,16 +167,22 @@ static_assert(kMixPts / 2 <= kTabPref, "the list of far points takes pref's spac
 static_assert(kWarps * kFineBins / 2 + SVPF_MAX_PARTICLES / 2 <= kTabPts + kTabPref && 4 * kMixPts <= kTabPts,
               "uses of the points' space");
 
-__host__ __device__ inline int fast_table_floats(bool mixture) {
-    return round_up(kTabBasis + kTabPts + kTabShorts / 2 + 8 + (mixture ? kTabPref + 2 * kMaxSrc : 0), 16);
+// Without the mixture the binning ranks of many particles extend the points' space.
+__host__ __device__ inline int fast_points_floats(int np, bool mixture) {
+    const int bins = kWarps * kFineBins / 2 + np / 2;
+    return mixture || bins < kTabPts ? kTabPts : bins;
+}
+__host__ __device__ inline int fast_table_floats(int np, bool mixture) {
+    return round_up(kTabBasis + fast_points_floats(np, mixture) + kTabShorts / 2 + 8 +
+                        (mixture ? kTabPref + 2 * kMaxSrc : 0), 16);
 }
 
-__device__ inline FastTab carve_fast(float* p, bool mixture) {
+__device__ inline FastTab carve_fast(float* p, int np, bool mixture) {
     FastTab t;
     t.basis = p;
     p += kTabBasis;
     t.pts = p;
-    p += kTabPts;
+    p += fast_points_floats(np, mixture);
     t.pref = t.src_x = t.src_w = nullptr;
     if (mixture) {
         t.pref = p;
@@ -231,14 +240,15 @@ __device__ __forceinline__ unsigned block_scan(unsigned own, unsigned& all, Fast
     return ex;
 }
 
-// Sorts the n coordinates x into fine bins, within a bin by particle, so that
+// Sorts the n coordinates x(i) into fine bins, within a bin by particle, so that
 // the order and with it every later sum is reproducible: xs[slot], pidx[slot]
 // (the particle) and fstart.  Each warp ranks its own stretch of particles
 // with match_any, two groups of 32 at a time.  (Shared-memory atomics and a
 // count of the smaller indices in the bin cost half as much again at
 // N = 4096.)  Ends with a barrier.
-__device__ inline void fast_bin(const float* x, int n, float fs, float* xs, unsigned short* pidx, const FastTab& t,
-                                FastSh& sh) {
+template <class FX>
+__device__ __forceinline__ void fast_bin(FX x, int n, float fs, float* xs, unsigned short* pidx, const FastTab& t,
+                                         FastSh& sh) {
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
     unsigned short* hist = reinterpret_cast<unsigned short*>(t.pts);     // [kWarps][kFineBins]
     unsigned short* rank = hist + kWarps * kFineBins;                    // by particle
@@ -254,7 +264,7 @@ __device__ inline void fast_bin(const float* x, int n, float fs, float* xs, unsi
     const unsigned below = (1u << lane) - 1u;
     for (int base = lo; base < hi; base += 64) {
         const int i0 = base + lane, i1 = i0 + 32;
-        const int f0 = i0 < hi ? fine_bin(x[i0], fs) : kFineBins, f1 = i1 < hi ? fine_bin(x[i1], fs) : kFineBins;
+        const int f0 = i0 < hi ? fine_bin(x(i0), fs) : kFineBins, f1 = i1 < hi ? fine_bin(x(i1), fs) : kFineBins;
         const unsigned m0 = __match_any_sync(0xffffffffu, f0), m1 = __match_any_sync(0xffffffffu, f1);
         int at = 0;
         if (i0 < hi) at = hw[f0];
@@ -301,7 +311,7 @@ __device__ inline void fast_bin(const float* x, int n, float fs, float* xs, unsi
     }
     __syncthreads();
     for (int i = lo + lane; i < hi; i += 32) {
-        const float v = x[i];
+        const float v = x(i);
         const int slot = hw[fine_bin(v, fs)] + rank[i];
         xs[slot] = v;
         pidx[slot] = (unsigned short)i;
@@ -498,10 +508,11 @@ __device__ __forceinline__ void fast_points(const float* __restrict__ xs, float 
 }
 
 // Sums at a panel's points -> Chebyshev coefficients, in place, one thread per
-// (panel, sum); sums are rows r0 .. r0 + nq - 1 of pts.
+// (panel, sum); sums are arrays r0 .. r0 + nq - 1 of STRIDE floats in pts.
+template <int STRIDE = kMaxPts>
 __device__ __forceinline__ void fast_coefficients(const FastTab& t, int nc, int r0, int nq) {
     for (int it = threadIdx.x; it < nc * nq; it += kThreads) {
-        float* v = t.pts + (size_t)(r0 + it / nc) * kMaxPts + (it % nc) * kP;
+        float* v = t.pts + (r0 + it / nc) * STRIDE + (it % nc) * kP;
         float a[kP];
 #pragma unroll
         for (int q = 0; q < kP; q += 4) *reinterpret_cast<float4*>(a + q) = *reinterpret_cast<const float4*>(v + q);
@@ -521,17 +532,17 @@ __device__ __forceinline__ void fast_coefficients(const FastTab& t, int nc, int 
     }
 }
 
-// Transport sums at the points (rows 4..10 of pts: sum K g, sum u K^2, then for
+// Transport sums at the points (arrays OUT.. of STRIDE floats in pts: sum K g, sum u K^2, then for
 // full Newton sum K, sum K c, sum K (3 - 4K), then for the KSD sum g u K^2 and
 // sum K^2 (3 - 4K)) over the points' weights.  Eight lanes share the columns of
 // two points: with 150 to 300 points that keeps every thread in work.
-template <bool FULL, bool KSD>
+template <bool FULL, bool KSD, int STRIDE = kMaxPts, int OUT = 4>
 __device__ __forceinline__ void fast_point_sums(const FastTab& t, int m, int m_pad) {
     constexpr int S = 8, R = 2;
     const float* __restrict__ X = t.pts;
-    const float* __restrict__ Q1 = t.pts + kMaxPts;
-    const float* __restrict__ QG = t.pts + 2 * kMaxPts;
-    const float* __restrict__ QC = t.pts + 3 * kMaxPts;
+    const float* __restrict__ Q1 = t.pts + STRIDE;
+    const float* __restrict__ QG = t.pts + 2 * STRIDE;
+    const float* __restrict__ QC = t.pts + 3 * STRIDE;
     const int grp = threadIdx.x / S, q = threadIdx.x % S;
     for (int base = 0; base < m; base += R * kThreads / S) {
         const int r0 = base + R * grp;
@@ -585,7 +596,7 @@ __device__ __forceinline__ void fast_point_sums(const FastTab& t, int m, int m_p
                 if ((k >= 2 && k < 5 && !FULL) || (k >= 5 && !KSD)) continue;
 #pragma unroll
                 for (int o = S / 2; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-                if (q == 0 && r0 + r < m) t.pts[(size_t)(4 + k) * kMaxPts + r0 + r] = v[k];
+                if (q == 0 && r0 + r < m) t.pts[(OUT + k) * STRIDE + r0 + r] = v[k];
             }
         }
     }

@@ -37,8 +37,13 @@ constexpr int kFastMinN = 257;
 // Bit of a filter's tile byte: its ticks go through the fast sums; the tile is
 // the one its sweeps use when the particles do not fit them.
 constexpr int kTileFast = 0x80;
+// Two-factor filters, 592 of one size, 40 Stein steps: 200 0.86 / 1.36 ms, 256
+// 1.05 / 1.47, 320 2.36 / 1.71, 512 3.45 / 2.12, 1024 13.0 / 3.26, 2048 50.9 /
+// 5.96.
+constexpr int kFastMinN2f = 257;
 SVPF_HD inline bool fast_tick(int n, const svpf_config_t& c) {
-    return n >= kFastMinN && !c.use_two_factor && !c.use_heun && !c.use_student_t_state &&
+    if (c.use_two_factor) return n >= kFastMinN2f;
+    return n >= kFastMinN && !c.use_heun && !c.use_student_t_state &&
            (!c.use_newton || c.use_full_newton);
 }
 
@@ -129,6 +134,7 @@ size_t tick_smem_bytes_batch(int n, const svpf_config_t& c, bool heun);
 // The single-filter kernel's: the tick's layout plus the pre-drawn SVLD normals.
 size_t tick_smem_bytes_single(int n, int C, bool heun);
 size_t tick_smem_bytes_2f(int n, int C);
+size_t tick_smem_bytes_2f_fast(int n);
 // Largest dynamic shared memory a CTA may use on the current device.
 size_t max_dyn_smem();
 // Current device index in [0, kMaxDevices), or -1.

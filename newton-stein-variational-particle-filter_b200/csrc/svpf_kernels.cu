@@ -13,6 +13,7 @@
 
 #include "svpf_internal.h"
 #include "svpf_tick.cuh"
+#include "svpf_tick2f.cuh"
 
 namespace svpf {
 
@@ -76,6 +77,7 @@ size_t tick_smem_bytes_batch(int n, const svpf_config_t& c, bool heun) {
 size_t tick_smem_bytes_single(int n, int C, bool heun) {
     return (size_t)(smem_floats(n, C, heun) + pre_floats(n, C)) * sizeof(float);
 }
+size_t tick_smem_bytes_2f_fast(int n) { return (size_t)fast_smem_floats_2f(n) * sizeof(float); }
 size_t tick_smem_bytes_2f(int n, int C) { return (size_t)smem_floats_2f(n, C) * sizeof(float); }
 
 // ---- per-device facts and kernel attributes --------------------------------

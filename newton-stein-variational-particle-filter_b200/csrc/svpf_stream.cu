@@ -110,14 +110,16 @@ BatchArgs round_args(svpf_stream* s) {
     return a;
 }
 
-// Two-factor filters with at least this many particles take a cluster of
-// kClusterMembers2f CTAs in the request loop: a round waits for its longest
-// tick, and one CTA needs ~30 ms for an N = 2048 two-factor tick of 40 Stein
-// steps.
+// Two-factor filters with at least this many particles that sweep over their
+// pairs take a cluster of kClusterMembers2f CTAs in the request loop: a round
+// waits for its longest tick, and one CTA needs ~30 ms to sweep an N = 2048
+// two-factor tick of 40 Stein steps.  (Through the fast sums one CTA needs
+// ~1 ms; only filters whose tables do not fit shared memory sweep.)
 constexpr int kClusterMinN = 1024;
 
 bool big_2f(const svpf_stream* s, int slot) {
-    return s->cfgs[slot].use_two_factor && s->ns[slot] >= kClusterMinN && s->grid2c > 0;
+    return s->cfgs[slot].use_two_factor && !(s->tiles[slot] & kTileFast) && s->ns[slot] >= kClusterMinN &&
+           s->grid2c > 0;
 }
 
 // One round: d_req[0, c1) single-factor slots, then c2 two-factor slots of
@@ -235,7 +237,11 @@ svpf_stream_t* svpf_stream_create(int max_instruments, size_t hbm_budget_bytes, 
         s->smem1 = tick_smem_bytes_batch(n_max, any, false);
         s->smem2 = tick_smem_bytes_2f(n_max, 1);
         if (s->smem1 <= max_dyn_smem()) s->grid1 = batch_grid(s->smem1);
-        if (s->smem2 <= max_dyn_smem()) s->grid2 = batch_grid_2f(s->smem2);
+        if (s->smem2 <= max_dyn_smem()) {
+            const size_t fast = tick_smem_bytes_2f_fast(n_max);
+            if (fast <= max_dyn_smem()) s->smem2 = std::max(s->smem2, fast);
+            s->grid2 = batch_grid_2f(s->smem2);
+        }
         s->smem2c = tick_smem_bytes_2f(n_max, kClusterMembers2f);
         if (n_max >= kClusterMinN && s->smem2c <= max_dyn_smem()) s->grid2c = batch_cluster_grid_2f(s->smem2c);
         ok = s->grid1 > 0 || s->grid2 > 0;
@@ -305,8 +311,10 @@ int svpf_stream_admit(svpf_stream_t* s, int n, const svpf_config_t* cfg, const S
     s->used_floats += (size_t)L;
     {
         const int t = tuned_batch_tile(n);
+        const bool fast = fast_tick(n, *cfg) && (!cfg->use_two_factor ||
+                                                 (s->grid2 > 0 && tick_smem_bytes_2f_fast(n) <= s->smem2));
         s->tiles[slot] = (uint8_t)((t >= kBatchTileLo && t <= kBatchTileHi ? t : default_batch_tile(n)) |
-                                   (fast_tick(n, *cfg) ? kTileFast : 0));
+                                   (fast ? kTileFast : 0));
     }
     // control record as svpf_initialize leaves it (svpf_optimized_graph.cu:349-451)
     svpf_config_t c = *cfg;

@@ -107,7 +107,7 @@ struct FastWork {
 // Floats of dynamic shared memory of a fast tick.
 __host__ __device__ inline int fast_smem_floats(int n) {
     const int np = round_up(n, 64);
-    return 3 * np + np / 2 + fast_table_floats(true);
+    return 3 * np + np / 2 + fast_table_floats(np, true);
 }
 
 // The scaled prior means (w.c) as points, once per tick, in panels of 0.75
@@ -123,7 +123,7 @@ __device__ inline bool fast_sources(FastWork& w, const Plan& pl, int n, FastSh& 
         w.src.up = wide ? 0.5f : 1.0f;
         w.src.near = wide ? 0 : 3;
         w.src.far2 = wide ? 5.0625f : 20.25f;
-        fast_bin(w.c, n, kFineScale * w.src.up, w.b, w.pidx, t, sh);
+        fast_bin([&](int i) { return w.c[i]; }, n, kFineScale * w.src.up, w.b, w.pidx, t, sh);
         const Panels p = fast_panels(3, t.src_pt, t.comp, kFineBins / kFine, kMaxSrc, true, t, sh);
         if (sh.over) {
             __syncthreads();   // everyone has read it
@@ -153,7 +153,7 @@ __device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_con
                                FastSh& sh, float& ksd) {
     const int tid = threadIdx.x, n = io.n;
     const FastTab& t = w.tab;
-    fast_bin(w.a, n, kFineScale, w.b, w.pidx, t, sh);
+    fast_bin([&](int i) { return w.a[i]; }, n, kFineScale, w.b, w.pidx, t, sh);
     const Panels p = fast_panels(3, t.pt, t.comp, kMaxComp, kMaxPts, false, t, sh);
     // the mixture's panels: the same ones unless they are too many sigma wide
     const Panels q = w.sft == 3 ? p : fast_panels(w.sft, t.mpt, t.mcomp, kMixComp, kMixPts, false, t, sh);
@@ -326,7 +326,7 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
         fw.b = sm.h[1];
         fw.c = sm.g;
         fw.pidx = reinterpret_cast<unsigned short*>(sm.c);
-        fw.tab = carve_fast(sm.c + sm.np / 2, true);
+        fw.tab = carve_fast(sm.c + sm.np / 2, sm.np, true);
         fast_load_tables(fw.tab);
     }
     if (tid == 0) {

@@ -93,13 +93,126 @@ __device__ inline void grad_pass_2f(const Smem2& sm, int cur, const Plan& pl, co
     }
 }
 
-template <int R, int S>
+// Workspace of the fast two-factor tick (one CTA): per factor the positions
+// (moved in place), g and the positions at tick start in the Smem2 view, and
+// shared by the factors the binned coordinates, their particles and the tables.
+struct FastWork2 {
+    float* xs;
+    unsigned short* pidx;
+    FastTab tab;
+};
+
+// Floats of dynamic shared memory of a fast two-factor tick.
+__host__ __device__ inline int fast_smem_floats_2f(int n) {
+    const int np = round_up(n, 64);
+    return 7 * np + np / 2 + fast_table_floats(np, false);
+}
+
+__device__ inline Smem2 carve_2f_fast(float* base, int n, FastWork2& w) {
+    Smem2 s;
+    const int np = round_up(n, 64);
+    for (int k = 0; k < 2; ++k) {
+        Smem& f = s.f[k];
+        float* b = base + 3 * k * np;
+        f.h[0] = f.h[1] = b;
+        f.g = b + np;
+        s.prev[k] = b + 2 * np;
+        f.c = f.mu = f.v = f.phi0 = f.phi1 = f.pre = nullptr;
+        f.n = n;
+        f.np = np;
+        f.m_len = f.p2 = f.Lp = 0;
+        f.row0 = 0;
+        f.row1 = n;
+    }
+    w.xs = base + 6 * np;
+    w.pidx = reinterpret_cast<unsigned short*>(base + 7 * np);
+    w.tab = carve_fast(base + 7 * np + np / 2, np, false);
+    return s;
+}
+
+// Vanilla transport of one factor through the fast sums (svpf_fast.cuh), in
+// place; v: the factor's RMSProp moments in global memory.  Positions stay in
+// log-volatility units; the sums run in bandwidths from the factor's mean.  A
+// step whose particles do not fit the tables sweeps over the pairs.
+__device__ inline void fast_transport_2f(const Smem& f, float* __restrict__ v, const FastWork2& w, const FactorPlan& fp,
+                                         const svpf_config_t& cfg, float beta, const Noise& nz, int kn, FastSh& sh) {
+    const int tid = threadIdx.x, n = f.n;
+    const FastTab& t = w.tab;
+    float* x = f.h[0];
+    const float* g = f.g;
+    const float ib = fp.inv_bw, cen = fp.center;
+    const float sign = cfg.stein_repulsive_sign == 1 ? 1.0f : -1.0f;
+    const float inv_n = 1.0f / (float)n, rr = cfg.rmsprop_rho;
+    const float es = fp.eps_step * beta;
+    // the row's new position from its sums
+    auto move = [&](int i, float kg, float gk) {
+        const float phi = (kg + sign * 2.0f * ib * gk) * inv_n;
+        const float vn = rr * v[i] + (1.0f - rr) * phi * phi;
+        v[i] = vn;
+        const float drift = es * phi * rsqrtf(vn + cfg.rmsprop_eps);
+        float diff = 0.0f;
+        if (fp.temp > 1e-6f) diff = sqrtf(2.0f * es * fp.temp) * nz.normal(i, kn);
+        return clamp_h(x[i] + drift + diff);
+    };
+    fast_bin([&](int i) { return (x[i] - cen) * ib; }, n, kFineScale, w.xs, w.pidx, t, sh);
+    const Panels p = fast_panels(3, t.pt, t.comp, kFineBins / kFine, kMaxPts2f, false, t, sh);
+    if (sh.over) {
+        for (int i = tid; i < n; i += kThreads) {
+            const float xi = x[i] * ib;
+            float kg = 0.0f, gk = 0.0f;
+            for (int j = 0; j < n; ++j) {
+                const float u = j == i ? 0.0f : fmaf(x[j], -ib, xi);
+                const float K = rcp_approx(fmaf(u, u, 1.0f));
+                kg = fmaf(K, g[j], kg);
+                gk = fmaf(u, K * K, gk);
+            }
+            w.xs[i] = move(i, kg, gk);
+        }
+        __syncthreads();
+        for (int i = tid; i < n; i += kThreads) x[i] = w.xs[i];
+        __syncthreads();
+        return;
+    }
+    const int m_pad = round_up(p.m, 32);
+    fast_points(w.xs, 1.0f, t, p, t.pts, m_pad, kHPad);
+    for (int i = p.m + tid; i < m_pad; i += kThreads) t.pts[kMaxPts2f + i] = t.pts[2 * kMaxPts2f + i] = 0.0f;
+    fast_weights<true, false, false>(w.xs, 1.0f, t, p, t.pts + kMaxPts2f, t.pts + 2 * kMaxPts2f, nullptr,
+                                     [&](int j) { return g[w.pidx[j]]; }, [](int) { return 0.0f; });
+    __syncthreads();
+    fast_point_sums<false, false, kMaxPts2f, 3>(t, p.m, m_pad);
+    __syncthreads();
+    fast_coefficients<kMaxPts2f>(t, p.nc, 3, 2);
+    __syncthreads();
+    for (int s = tid; s < n; s += kThreads) {
+        const float u = w.xs[s];
+        const int i = w.pidx[s];
+        const int b = fine_bin(u) / kFine;
+        const int j0 = t.fstart[kFine * b];
+        const float* row = t.pts + 3 * kMaxPts2f + p.pt[b];
+        float kg, gk;
+        if (p.interpolated(b, t.fstart[kFine * (b + 1)] - j0)) {
+            float T[kP];
+            cheb(p.local(u, b), T);
+            kg = cheb_dot(T, row);
+            gk = cheb_dot(T, row + kMaxPts2f);
+        } else {
+            kg = row[s - j0];
+            gk = row[kMaxPts2f + s - j0];
+        }
+        x[i] = move(i, kg, gk);
+    }
+    __syncthreads();
+}
+
+// FAST: the transports go through the fast sums (one CTA; sm from carve_2f_fast).
+template <int R, int S, bool FAST = false>
 __device__ void run_tick_2f(const svpf_config_t& cfg, const SVPFParams& prm, svpf_ctl_t& ctl, float y_t,
                             float y_prev, const FilterIO& io, const Noise& nz, const Smem2& sm, Plan& pl,
-                            const Team& team, svpf_out_t& out) {
+                            const Team& team, svpf_out_t& out, const FastWork2* fw = nullptr, FastSh* fsh = nullptr) {
     const int tid = threadIdx.x;
     const int n = io.n;
     const int np = sm.f[0].np;
+    if constexpr (FAST) fast_load_tables(fw->tab);
     if (tid == 0) {
         pl.flag = 0;
         make_plan_2f(cfg, prm, ctl, y_t, y_prev, pl);
@@ -177,7 +290,7 @@ __device__ void run_tick_2f(const svpf_config_t& cfg, const SVPFParams& prm, svp
     __syncthreads();
     // ---- own rows' RMSProp state (positions stay in log-volatility units)
     const int row0 = sm.f[0].row0, nloc = sm.f[0].row1 - row0;
-    for (int li = tid; li < nloc; li += kThreads) {
+    for (int li = tid; !FAST && li < nloc; li += kThreads) {
         sm.f[0].v[li] = io.v[row0 + li];
         sm.f[1].v[li] = io.v[n + row0 + li];
     }
@@ -195,15 +308,20 @@ __device__ void run_tick_2f(const svpf_config_t& cfg, const SVPFParams& prm, svp
             const bool last = it == pl.budget - 1;
             grad_pass_2f(sm, cur, pl, cfg, prm, beta, (last && team.rank == 0) ? io.lw : nullptr);
             __syncthreads();
-            transport_pass<R, S, 0, false, kTransport>(sm.f[0], cur, pl.fac[0], cfg, beta, nz, kn, team);
-            transport_pass<R, S, 0, false, kTransport>(sm.f[1], cur, pl.fac[1], cfg, beta, nz, kn + 1, team);
-            team.sync();
-            cur ^= 1;
+            if constexpr (FAST) {
+                fast_transport_2f(sm.f[0], io.v, *fw, pl.fac[0], cfg, beta, nz, kn, *fsh);
+                fast_transport_2f(sm.f[1], io.v + n, *fw, pl.fac[1], cfg, beta, nz, kn + 1, *fsh);
+            } else {
+                transport_pass<R, S, 0, false, kTransport>(sm.f[0], cur, pl.fac[0], cfg, beta, nz, kn, team);
+                transport_pass<R, S, 0, false, kTransport>(sm.f[1], cur, pl.fac[1], cfg, beta, nz, kn + 1, team);
+                team.sync();
+                cur ^= 1;
+            }
             if (pl.temp > 1e-6f) kn += 2;
         }
     }
 
-    for (int li = tid; li < nloc; li += kThreads) {
+    for (int li = tid; !FAST && li < nloc; li += kThreads) {
         io.v[row0 + li] = sm.f[0].v[li];
         io.v[n + row0 + li] = sm.f[1].v[li];
     }

@@ -94,3 +94,56 @@ def test_fast_sums_match_oracle(pkg, oracle_mod, newton, sigma):
             dev = max(abs(getattr(a[f], name) - w) for a in around) / max(1.0, abs(w))
             assert abs(value - w) < max(base, 4 * dev) * max(1.0, abs(w)), (tag, name, value, w, dev)
     b.close()
+
+
+@pytest.mark.parametrize("exact", [1, 0])
+def test_two_factor_fast_sums_match_oracle(pkg, oracle_mod, exact):
+    """The same for the two-factor tick's transports: both factors of made
+    states, a spread of the slow factor over its floored bandwidth included
+    (its step sweeps over the pairs)."""
+    sizes = [257, 300, 513, 1025, 2048]
+    kinds2 = ["cloud", "point", "outliers", "clamped", "spread"]
+    ns = [n for n in sizes for _ in kinds2] + [4096]
+    kinds = kinds2 * len(sizes) + ["outliers"]
+    F, n_max = len(ns), max(ns)
+    cfg = pkg.default_config(2, 6.0)
+    cfg.update(use_two_factor=1, rho_fast=0.80, sigma_fast=0.30, rho_slow=0.97, sigma_slow=0.10, bw_floor_fast=0.01,
+               bw_floor_slow=0.05, use_svld=1, use_annealing=1, n_anneal_steps=3, temperature=0.45, use_mim=1,
+               mim_jump_prob=0.25, mim_jump_scale=9.0, use_guide=1, guide_strength=0.12, use_exact_gradient=exact)
+    params = [(0.95, 0.1, -3.0, 0.0)] * F
+    b = pkg.Batch(ns, [cfg] * F, [pkg.Params(*p) for p in params])
+    b.initialize(seed=3)
+    rng = np.random.default_rng(23)
+    for f in range(F):
+        ctl = b.get_state(f)[0]
+        h = np.concatenate([_state(kinds[f], ns[f], rng, 0.0), _state(kinds[f], ns[f], rng, 0.2)])
+        v = rng.uniform(0.05, 0.5, 2 * ns[f]).astype(np.float32)
+        b.set_state(f, ctl, h, (h - 0.1).astype(np.float32), v, np.zeros(ns[f], np.float32))
+    y = (0.2 + 0.02 * np.arange(F)).astype(np.float32)
+    nrm, uni = tape.tape(9, 0, n_max, 24, 2)
+    b.set_noise_tape(nrm, uni)
+    yp = np.zeros(F, np.float32)
+    twins = [_twin(oracle_mod, b, f, cfg, params[f]) for f in range(F)]
+    mirrors = []
+    for nudge in (0.0, 2.0 ** -22, -(2.0 ** -22)):
+        m = [_twin(oracle_mod, b, f, cfg, params[f], 1) for f in range(F)]
+        for o in m:
+            o.h = o.h * (1.0 + nudge)
+        mirrors.append(m)
+    ll, vol, hm = b.step(y, yp)
+    ctl = b.ctl()
+    with cf.ThreadPoolExecutor(max_workers=min(16, os.cpu_count() or 1)) as pool:
+        def step(m):
+            return list(pool.map(lambda f: m[f].step(y[f], yp[f], nrm[:, :ns[f]], uni[:, :ns[f]]), range(F)))
+        want, around = step(twins), [step(m) for m in mirrors]
+    for f in range(F):
+        tag = (kinds[f], ns[f])
+        assert ctl[f].status == 0, tag
+        dev = max(rel_err(m[f].h, twins[f].h) for m in mirrors)
+        got = b.get_particles(f)
+        assert rel_err(got, twins[f].h) < max(TOL, 4 * dev), (tag, rel_err(got, twins[f].h), dev)
+        for name, value in (("loglik", ll[f]), ("vol", vol[f]), ("h_mean", hm[f])):
+            w = getattr(want[f], name)
+            dev = max(abs(getattr(a[f], name) - w) for a in around) / max(1.0, abs(w))
+            assert abs(value - w) < max(TOL, 4 * dev) * max(1.0, abs(w)), (tag, name, value, w, dev)
+    b.close()
