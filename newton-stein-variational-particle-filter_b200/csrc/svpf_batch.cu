@@ -61,6 +61,7 @@ struct svpf_batch {
     unsigned long long seed = 0;
     size_t smem = 0, smem2 = 0;
     int grid = 0, grid2 = 0;
+    bool wide = false, wide2 = false;   // on wide CTAs (WideChoice)
     int launches = 0;
     int heun = 0;
     int prod = 0;                // every single-factor filter has the production configuration
@@ -126,14 +127,14 @@ int enqueue_tick(svpf_batch* b, const float* d_yt, const float* d_yp, svpf_out_t
     if (cudaMemsetAsync(b->d_queue, 0, 2 * sizeof(int), b->stream) != cudaSuccess) return SVPF_ERR_CUDA;
     BatchArgs a = make_args(b, d_yt, d_yp, d_out);
     if (b->F1 > 0) {
-        if (launch_batch(a, b->smem, b->grid, b->stream) != cudaSuccess) return SVPF_ERR_CUDA;
+        if (launch_batch(a, b->smem, b->grid, b->wide, b->stream) != cudaSuccess) return SVPF_ERR_CUDA;
         ++b->launches;
     }
     if (b->F2 > 0) {
         a.F = b->F2;
         a.order = b->d_order + b->F1;
         a.queue = b->d_queue + 1;
-        if (launch_batch_2f(a, b->smem2, b->grid2, b->stream) != cudaSuccess) return SVPF_ERR_CUDA;
+        if (launch_batch_2f(a, b->smem2, b->grid2, b->wide2, b->stream) != cudaSuccess) return SVPF_ERR_CUDA;
         ++b->launches;
     }
     return SVPF_OK;
@@ -146,6 +147,19 @@ void drop_graph(svpf_batch* b) {
     b->graph = nullptr;
 }
 
+uint8_t tile_code(const svpf_batch* b, int f) { return (uint8_t)(b->tiles[f] | (b->fast[f] ? kTileFast : 0)); }
+
+// CTA shape and grid of each kernel, from the filters' tiles.
+bool choose_grids(svpf_batch* b) {
+    WideChoice w, w2;
+    for (int f = 0; f < b->F; ++f) (b->tf[f] ? w2 : w).add(b->ns[f], b->cfgs[f], tile_code(b, f));
+    b->wide = w.wide();
+    b->wide2 = w2.wide();
+    if (b->F1 > 0) b->grid = batch_grid(b->smem, b->wide);
+    if (b->F2 > 0) b->grid2 = batch_grid_2f(b->smem2, b->wide2);
+    return (b->F1 == 0 || b->grid > 0) && (b->F2 == 0 || b->grid2 > 0);
+}
+
 int upload_tiles(svpf_batch* b) {
     std::vector<uint8_t> code(b->F);
     for (int f = 0; f < b->F; ++f) {
@@ -154,7 +168,7 @@ int upload_tiles(svpf_batch* b) {
         // (a two-factor filter's tables may not fit where its sweeps do)
         b->fast[f] = fast_tick(b->ns[f], b->cfgs[f]) &&
                      (!b->tf[f] || tick_smem_bytes_2f_fast(b->ns[f]) <= max_dyn_smem());
-        code[f] = (uint8_t)(b->tiles[f] | (b->fast[f] ? kTileFast : 0));
+        code[f] = tile_code(b, f);
     }
     return cudaMemcpy(b->d_tile, code.data(), b->F, cudaMemcpyHostToDevice) == cudaSuccess ? SVPF_OK : SVPF_ERR_CUDA;
 }
@@ -247,18 +261,13 @@ svpf_batch_t* svpf_batch_create(int F, const int* ns, const svpf_config_t* cfgs,
          cudaMemcpy(b->d_ctl, ctl.data(), F * sizeof(svpf_ctl_t), cudaMemcpyHostToDevice) == cudaSuccess &&
          cudaMemset(b->d_lw, 0, b->total * sizeof(float)) == cudaSuccess;
     ok = ok && upload_tiles(b) == SVPF_OK;
-    if (ok && b->F1 > 0) {
-        b->smem = smem1;
-        b->grid = batch_grid(b->smem);
-        ok = b->grid > 0;
-    }
-    if (ok && b->F2 > 0) {
+    b->smem = smem1;
+    if (b->F2 > 0) {
         b->smem2 = tick_smem_bytes_2f(n_max2, 1);
         for (int f = 0; f < F; ++f)
             if (b->tf[f] && b->fast[f]) b->smem2 = std::max(b->smem2, tick_smem_bytes_2f_fast(ns[f]));
-        b->grid2 = batch_grid_2f(b->smem2);
-        ok = b->grid2 > 0;
     }
+    ok = ok && choose_grids(b);
     if (!ok) {
         svpf_batch_destroy(b);
         return nullptr;
@@ -578,6 +587,8 @@ int tune_one(int n, int ticks, int* best_tile) {
     std::vector<SVPFParams> pv(F, SVPFParams{0.97f, 0.15f, -1.0f, 0.0f});
     svpf_batch_t* b = svpf_batch_create(F, nv.data(), cv.data(), pv.data(), nullptr);
     if (!b) return SVPF_ERR_CUDA;
+    b->wide = false;   // the tiles' own kernel
+    b->grid = batch_grid(b->smem);
     float* d_y = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     int rc = svpf_batch_initialize(b, 1234);
@@ -646,6 +657,7 @@ int svpf_batch_set_tile(svpf_batch_t* b, int f, int R, int S) {
     b->tiles[f] = (uint8_t)tile;
     b->fast[f] = 0;   // a forced tile is the one that runs
     drop_graph(b);
+    if (!choose_grids(b)) return SVPF_ERR_CUDA;
     return cudaMemcpy(b->d_tile + f, &b->tiles[f], 1, cudaMemcpyHostToDevice) == cudaSuccess ? SVPF_OK
                                                                                           : SVPF_ERR_CUDA;
 }

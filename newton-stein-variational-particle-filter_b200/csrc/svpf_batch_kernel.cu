@@ -13,13 +13,17 @@ __device__ __forceinline__ void copy_words(T* dst, const T* src) {
     static_assert(sizeof(T) % 4 == 0, "word copy");
     const int* s = reinterpret_cast<const int*>(src);
     int* d = reinterpret_cast<int*>(dst);
-    for (int k = threadIdx.x; k < (int)(sizeof(T) / 4); k += kThreads) d[k] = s[k];
+    for (int k = threadIdx.x; k < (int)(sizeof(T) / 4); k += blockDim.x) d[k] = s[k];
 }
 
 // PROD: launched only when every single-factor filter of the batch has the
 // production configuration (a.prod), so only its code paths are compiled.
-template <bool PROD>
-__global__ void __launch_bounds__(kThreads, 2) batch_tick_kernel(const __grid_constant__ BatchArgs a) {
+// NT threads per CTA: two CTAs of 256 per SM, or one of 512 (wide), which
+// shortens a filter's tick and is launched when the largest ticks, not the
+// number of filters, make the launch long; its filters go through the fast
+// sums or have at most 256 particles (tiles with one row per thread).
+template <bool PROD, int NT>
+__global__ void __launch_bounds__(NT, 2 * kThreads / NT) batch_tick_kernel(const __grid_constant__ BatchArgs a) {
     extern __shared__ __align__(16) float smem[];
     __shared__ Plan pl;
     __shared__ svpf_ctl_t ctl;
@@ -57,13 +61,21 @@ __global__ void __launch_bounds__(kThreads, 2) batch_tick_kernel(const __grid_co
             const float ypr = readable_y_prev(yp);
             const int tile = a.tile[f];
             if (tile & kTileFast) {
-                run_tick<2, 1, false, PROD, 0, true>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out, &fsh);
-            } else switch (tile) {
-                case 1: run_tick<1, 4, false, PROD>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
-                case 2: run_tick<1, 2, false, PROD>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
-                case 3: run_tick<1, 1, false, PROD>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
-                case 4: run_tick<2, 1, false, PROD>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
-                default: run_tick<4, 1, false, PROD>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
+                run_tick<2, 1, false, PROD, 0, true, NT>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out, &fsh);
+            } else if constexpr (NT == kThreads) {
+                switch (tile) {
+                    case 1: run_tick<1, 4, false, PROD>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
+                    case 2: run_tick<1, 2, false, PROD>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
+                    case 3: run_tick<1, 1, false, PROD>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
+                    case 4: run_tick<2, 1, false, PROD>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
+                    default: run_tick<4, 1, false, PROD>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
+                }
+            } else {
+                switch (tile) {
+                    case 1: run_tick<1, 4, false, PROD, 0, false, NT>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
+                    case 2: run_tick<1, 2, false, PROD, 0, false, NT>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
+                    default: run_tick<1, 1, false, PROD, 0, false, NT>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
+                }
             }
             flag_y_prev(yp, ctl);
         }
@@ -76,7 +88,8 @@ __global__ void __launch_bounds__(kThreads, 2) batch_tick_kernel(const __grid_co
 }
 
 // Two-factor filters (their particle segments hold [fast (n); slow (n)]).
-__global__ void __launch_bounds__(kThreads, 2) batch_tick_2f_kernel(const __grid_constant__ BatchArgs a) {
+template <int NT>
+__global__ void __launch_bounds__(NT, 2 * kThreads / NT) batch_tick_2f_kernel(const __grid_constant__ BatchArgs a) {
     extern __shared__ __align__(16) float smem[];
     __shared__ Plan pl;
     __shared__ svpf_ctl_t ctl;
@@ -110,13 +123,21 @@ __global__ void __launch_bounds__(kThreads, 2) batch_tick_2f_kernel(const __grid
         if (!refuse_nonfinite(yt, ctl, out)) {   // a refused tick leaves the filter as it was
             const float ypr = readable_y_prev(yp);
             if (tile & kTileFast) {
-                run_tick_2f<1, 1, true>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out, &fw, &fsh);
-            } else switch (tile) {
-                case 1: run_tick_2f<1, 4>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
-                case 2: run_tick_2f<1, 2>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
-                case 3: run_tick_2f<1, 1>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
-                case 4: run_tick_2f<2, 1>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
-                default: run_tick_2f<4, 1>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
+                run_tick_2f<1, 1, true, NT>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out, &fw, &fsh);
+            } else if constexpr (NT == kThreads) {
+                switch (tile) {
+                    case 1: run_tick_2f<1, 4>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
+                    case 2: run_tick_2f<1, 2>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
+                    case 3: run_tick_2f<1, 1>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
+                    case 4: run_tick_2f<2, 1>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
+                    default: run_tick_2f<4, 1>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
+                }
+            } else {
+                switch (tile) {
+                    case 1: run_tick_2f<1, 4, false, NT>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
+                    case 2: run_tick_2f<1, 2, false, NT>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
+                    default: run_tick_2f<1, 1, false, NT>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
+                }
             }
             flag_y_prev(yp, ctl);
         }
@@ -226,45 +247,71 @@ cudaError_t launch_batch_2f_cluster(const BatchArgs& a, size_t smem_bytes, int g
     return cudaLaunchKernelEx(&cfg, kern, a);
 }
 
-int batch_grid_2f(size_t smem_bytes) {
-    if (configure_kernel((const void*)batch_tick_2f_kernel, (int)max_dyn_smem(), false) != cudaSuccess) {
+// CTAs of a kernel that can be resident at once on the current device.
+static int resident_ctas(const void* kern, int threads, size_t smem_bytes) {
+    if (configure_kernel(kern, (int)max_dyn_smem(), false) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_tick_2f_kernel, kThreads, smem_bytes);
-    if (per_sm < 1) return 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem_bytes);
     return sms * per_sm;
 }
 
-cudaError_t launch_batch_2f(const BatchArgs& a, size_t smem_bytes, int grid, cudaStream_t s) {
+int batch_grid_2f(size_t smem_bytes, bool wide) {
+    return wide ? resident_ctas((const void*)batch_tick_2f_kernel<kWideThreads>, kWideThreads, smem_bytes)
+                : resident_ctas((const void*)batch_tick_2f_kernel<kThreads>, kThreads, smem_bytes);
+}
+
+cudaError_t launch_batch_2f(const BatchArgs& a, size_t smem_bytes, int grid, bool wide, cudaStream_t s) {
     if (grid < 1) return cudaErrorInvalidConfiguration;
-    batch_tick_2f_kernel<<<grid, kThreads, smem_bytes, s>>>(a);
+    if (wide) batch_tick_2f_kernel<kWideThreads><<<grid, kWideThreads, smem_bytes, s>>>(a);
+    else batch_tick_2f_kernel<kThreads><<<grid, kThreads, smem_bytes, s>>>(a);
     return cudaGetLastError();
 }
 
-int batch_grid(size_t smem_bytes) {
-    if (configure_kernel((const void*)batch_tick_kernel<false>, (int)max_dyn_smem(), false) != cudaSuccess ||
-        configure_kernel((const void*)batch_tick_kernel<true>, (int)max_dyn_smem(), false) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
+int batch_grid(size_t smem_bytes, bool wide) {
+    const void* any = wide ? (const void*)batch_tick_kernel<false, kWideThreads> : (const void*)batch_tick_kernel<false, kThreads>;
+    const void* prod = wide ? (const void*)batch_tick_kernel<true, kWideThreads> : (const void*)batch_tick_kernel<true, kThreads>;
+    const int threads = wide ? kWideThreads : kThreads;
+    // both variants are bounded to the same number of CTAs per SM by their launch bounds
+    return resident_ctas(prod, threads, smem_bytes) > 0 ? resident_ctas(any, threads, smem_bytes) : 0;
+}
+
+cudaError_t launch_batch(const BatchArgs& a, size_t smem_bytes, int grid, bool wide, cudaStream_t s) {
+    if (grid < 1) return cudaErrorInvalidConfiguration;
+    if (wide) {
+        if (a.prod) batch_tick_kernel<true, kWideThreads><<<grid, kWideThreads, smem_bytes, s>>>(a);
+        else batch_tick_kernel<false, kWideThreads><<<grid, kWideThreads, smem_bytes, s>>>(a);
+    } else {
+        if (a.prod) batch_tick_kernel<true, kThreads><<<grid, kThreads, smem_bytes, s>>>(a);
+        else batch_tick_kernel<false, kThreads><<<grid, kThreads, smem_bytes, s>>>(a);
     }
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // both variants are bounded to 2 CTAs per SM by their launch bounds
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_tick_kernel<false>, kThreads, smem_bytes);
-    if (per_sm < 1) return 0;
-    return sms * per_sm;
-}
-
-cudaError_t launch_batch(const BatchArgs& a, size_t smem_bytes, int grid, cudaStream_t s) {
-    if (grid < 1) return cudaErrorInvalidConfiguration;
-    if (a.prod) batch_tick_kernel<true><<<grid, kThreads, smem_bytes, s>>>(a);
-    else batch_tick_kernel<false><<<grid, kThreads, smem_bytes, s>>>(a);
     return cudaGetLastError();
 }
+
+// Expected length of a list of ticks relative to one another: a fast tick's
+// phases grow slowly with n (a fixed part worth about 860 particles, 400 for a
+// two-factor tick), small filters sweep.
+static double tick_length(int n, const svpf_config_t& c) {
+    const bool tf = c.use_two_factor != 0;
+    const double its = tf ? 2.0 * (c.use_annealing ? c.n_anneal_steps : 1) * c.n_stein_steps : c.stein_max_steps;
+    return its * (n + (tf ? 400.0 : 860.0));
+}
+
+WideChoice::WideChoice() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        sms = 1;
+}
+void WideChoice::add(int n, const svpf_config_t& c, int tile) {
+    const double t = tick_length(n, c);
+    sum += t;
+    longest = t > longest ? t : longest;
+    if (!(tile & kTileFast) && (tile > 3 || n > kThreads || c.use_heun)) ok = false;
+}
+bool WideChoice::wide() const { return ok && sum < kWideLoad * sms * longest; }
 
 }  // namespace svpf

@@ -165,7 +165,7 @@ struct Plan {
     FactorPlan fac[2];     // two-factor: fast, slow
     float fmean[2];        // two-factor: factor means of the previous tick (guide)
     float gmean2[2];       // two-factor: EKF guide means
-    float red[5][kWarps];  // block reduction scratch
+    float red[5][16];      // block reduction scratch, a value per warp
     float ksd_slot[kMaxCluster];
 };
 
@@ -321,7 +321,7 @@ __device__ __forceinline__ float warp_min(float v) {
 
 // Reduce up to five values (op per slot: 0 sum, 1 max, 2 min); result visible
 // to all threads.  Contains two __syncthreads.
-template <int K>
+template <int K, int NT = kThreads>
 __device__ __forceinline__ void block_reduce(float (&v)[K], const int (&op)[K], Plan& pl) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
@@ -333,7 +333,7 @@ __device__ __forceinline__ void block_reduce(float (&v)[K], const int (&op)[K], 
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         float a = pl.red[k][0];
-        for (int i = 1; i < kWarps; ++i) {
+        for (int i = 1; i < NT / 32; ++i) {
             const float b = pl.red[k][i];
             a = op[k] == 0 ? a + b : op[k] == 1 ? fmaxf(a, b) : fminf(a, b);
         }
@@ -348,7 +348,7 @@ __device__ __forceinline__ void block_reduce(float (&v)[K], const int (&op)[K], 
 __device__ inline void bitonic_sort(float* m, int P) {
     for (int k = 2; k <= P; k <<= 1) {
         for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < P; i += kThreads) {
+            for (int i = threadIdx.x; i < P; i += blockDim.x) {
                 const int ixj = i ^ j;
                 if (ixj > i) {
                     const float a = m[i], b = m[ixj];

@@ -53,6 +53,8 @@
 
 namespace svpf {
 
+constexpr int kMaxWarps = 16;       // CTAs of 8 or 16 warps
+constexpr int kBinWarps = 8;        // warps that rank particles
 constexpr int kP = 12;              // points of a panel
 constexpr int kFine = 8;            // fine bins of a transport panel
 constexpr int kFineBins = 1024;
@@ -152,7 +154,7 @@ struct FastTab {
 };
 // Static shared scalars.
 struct FastSh {
-    unsigned scan[kWarps];
+    unsigned scan[kMaxWarps];
     int over;                 // points do not fit
     int n_far;                // mixture points far from every mean, listed in pref's space
 };
@@ -164,12 +166,12 @@ constexpr int kTabShorts = (kFineBins + 8) + (kFineBins / kFine + 8) + 2 * (kFin
                            2 * kMixComp;
 // binning counters and ranks take the points' space and the one behind it
 static_assert(kMixPts / 2 <= kTabPref, "the list of far points takes pref's space");
-static_assert(kWarps * kFineBins / 2 + SVPF_MAX_PARTICLES / 2 <= kTabPts + kTabPref && 4 * kMixPts <= kTabPts,
+static_assert(kBinWarps * kFineBins / 2 + SVPF_MAX_PARTICLES / 2 <= kTabPts + kTabPref && 4 * kMixPts <= kTabPts,
               "uses of the points' space");
 
 // Without the mixture the binning ranks of many particles extend the points' space.
 __host__ __device__ inline int fast_points_floats(int np, bool mixture) {
-    const int bins = kWarps * kFineBins / 2 + np / 2;
+    const int bins = kBinWarps * kFineBins / 2 + np / 2;
     return mixture || bins < kTabPts ? kTabPts : bins;
 }
 __host__ __device__ inline int fast_table_floats(int np, bool mixture) {
@@ -210,7 +212,7 @@ __device__ inline FastTab carve_fast(float* p, int np, bool mixture) {
 }
 
 __device__ __forceinline__ void fast_load_tables(const FastTab& t) {
-    for (int i = threadIdx.x; i < kP * kP + kP; i += kThreads) t.basis[i] = i < kP * kP ? kBasis[i] : kNode[i - kP * kP];
+    for (int i = threadIdx.x; i < kP * kP + kP; i += blockDim.x) t.basis[i] = i < kP * kP ? kBasis[i] : kNode[i - kP * kP];
 }
 
 // Fine bin of coordinate x; outliers share the first and the last bin, NaN the first.
@@ -231,8 +233,7 @@ __device__ __forceinline__ unsigned block_scan(unsigned own, unsigned& all, Fast
     __syncthreads();
     unsigned ex = inc - own;
     all = 0u;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
         const unsigned v = sh.scan[w];
         if (w < wp) ex += v;
         all += v;
@@ -244,22 +245,22 @@ __device__ __forceinline__ unsigned block_scan(unsigned own, unsigned& all, Fast
 // the order and with it every later sum is reproducible: xs[slot], pidx[slot]
 // (the particle) and fstart.  Each warp ranks its own stretch of particles
 // with match_any, two groups of 32 at a time.  (Shared-memory atomics and a
-// count of the smaller indices in the bin cost half as much again at
-// N = 4096.)  Ends with a barrier.
+// count of the smaller indices in the bin took twice as long at N = 4096; a
+// ballot per bit instead of match_any 5 % longer.)  Ends with a barrier.
 template <class FX>
 __device__ __forceinline__ void fast_bin(FX x, int n, float fs, float* xs, unsigned short* pidx, const FastTab& t,
                                          FastSh& sh) {
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-    unsigned short* hist = reinterpret_cast<unsigned short*>(t.pts);     // [kWarps][kFineBins]
-    unsigned short* rank = hist + kWarps * kFineBins;                    // by particle
+    unsigned short* hist = reinterpret_cast<unsigned short*>(t.pts);     // [kBinWarps][kFineBins]
+    unsigned short* rank = hist + kBinWarps * kFineBins;                    // by particle
     {
         uint4* h4 = reinterpret_cast<uint4*>(hist);
-        for (int i = tid; i < kWarps * kFineBins / 8; i += kThreads) h4[i] = make_uint4(0u, 0u, 0u, 0u);
+        for (int i = tid; i < kBinWarps * kFineBins / 8; i += blockDim.x) h4[i] = make_uint4(0u, 0u, 0u, 0u);
     }
     if (tid == 0) sh.over = sh.n_far = 0;
     __syncthreads();
-    const int per = round_up((n + kWarps - 1) / kWarps, 32);
-    const int lo = min(wp * per, n), hi = min(lo + per, n);
+    const int per = round_up((n + kBinWarps - 1) / kBinWarps, 32);
+    const int lo = min(wp * per, n), hi = wp < kBinWarps ? min(lo + per, n) : lo;
     unsigned short* hw = hist + wp * kFineBins;
     const unsigned below = (1u << lane) - 1u;
     for (int base = lo; base < hi; base += 64) {
@@ -284,10 +285,12 @@ __device__ __forceinline__ void fast_bin(FX x, int n, float fs, float* xs, unsig
     }
     __syncthreads();
     {
-        // four fine bins per thread: the warps' counts become their first slots
+        // four fine bins for each of 256 threads: the warps' counts become their first slots
+        const bool on = tid < kFineBins / 4;
         unsigned c4[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
+        for (int w = 0; w < kBinWarps; ++w) {
+            if (!on) break;
             const ushort4 v = reinterpret_cast<const ushort4*>(hist + w * kFineBins)[tid];
             c4[0] += v.x; c4[1] += v.y; c4[2] += v.z; c4[3] += v.w;
         }
@@ -295,13 +298,15 @@ __device__ __forceinline__ void fast_bin(FX x, int n, float fs, float* xs, unsig
         unsigned first = block_scan(c4[0] + c4[1] + c4[2] + c4[3], all, sh);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
+            if (!on) break;
             t.fstart[4 * tid + j] = (unsigned short)first;
             const unsigned next = first + c4[j];
             c4[j] = first;
             first = next;
         }
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
+        for (int w = 0; w < kBinWarps; ++w) {
+            if (!on) break;
             ushort4* h = reinterpret_cast<ushort4*>(hist + w * kFineBins) + tid;
             const ushort4 v = *h;
             *h = make_ushort4(c4[0], c4[1], c4[2], c4[3]);
@@ -310,9 +315,9 @@ __device__ __forceinline__ void fast_bin(FX x, int n, float fs, float* xs, unsig
         if (tid == 0) t.fstart[kFineBins] = (unsigned short)n;
     }
     __syncthreads();
-    for (int i = lo + lane; i < hi; i += 32) {
+    for (int i = tid; i < n; i += blockDim.x) {
         const float v = x(i);
-        const int slot = hw[fine_bin(v, fs)] + rank[i];
+        const int slot = hist[i / per * kFineBins + fine_bin(v, fs)] + rank[i];
         xs[slot] = v;
         pidx[slot] = (unsigned short)i;
     }
@@ -329,7 +334,7 @@ __device__ inline Panels fast_panels(int sft, unsigned short* pt, unsigned short
     p.sft = sft;
     p.narrow = (float)kFine / (float)(1 << sft);
     const int np = kFineBins >> sft;
-    const int per = np > kThreads ? np / kThreads : 1;   // panels per thread
+    const int per = np > kThreads ? np / kThreads : 1;   // panels per thread (of the first 256)
     const int b0 = threadIdx.x * per;
     unsigned own = 0u;   // interpolated panels, and from bit 16 points kept as they are
     if (b0 < np) {
@@ -391,7 +396,7 @@ __device__ __forceinline__ void fast_weights(const float* __restrict__ xs, float
                                              float* __restrict__ q1, float* __restrict__ qg, float* __restrict__ qc,
                                              FG gv, FC cv) {
     const int tid = threadIdx.x;
-    for (int base = 0; base < p.nc * kFine; base += kThreads) {
+    for (int base = 0; base < p.nc * kFine; base += (int)blockDim.x) {
         const int item = base + tid;
         const bool on = item < p.nc * kFine;
         const int s = item % kFine;
@@ -476,7 +481,7 @@ __device__ __forceinline__ void fast_weights(const float* __restrict__ xs, float
             }
         }
     }
-    for (int b = tid; b < kFineBins / kFine; b += kThreads) {
+    for (int b = tid; b < kFineBins / kFine; b += (int)blockDim.x) {
         const int j0 = t.fstart[kFine * b], cnt = t.fstart[kFine * (b + 1)] - j0;
         if (cnt == 0 || p.interpolated(b, cnt)) continue;
         const int o = p.pt[b];
@@ -494,24 +499,24 @@ __device__ __forceinline__ void fast_points(const float* __restrict__ xs, float 
                                             float* __restrict__ px, int m_pad, float far) {
     const float* node = t.basis + kP * kP;
     const float sc = (1.0f / p.narrow) * (1.0f / up), dn = 1.0f / up;
-    for (int i = threadIdx.x; i < kP * p.nc; i += kThreads) {
+    for (int i = threadIdx.x; i < kP * p.nc; i += (int)blockDim.x) {
         const int b = p.comp[i / kP], q = i % kP;
         px[p.pt[b] + q] = fmaf(node[q], sc, p.centre(b) * dn);
     }
-    for (int b = threadIdx.x; b < kFineBins >> p.sft; b += kThreads) {
+    for (int b = threadIdx.x; b < kFineBins >> p.sft; b += (int)blockDim.x) {
         const int j0 = t.fstart[b << p.sft], cnt = t.fstart[(b + 1) << p.sft] - j0;
         if (cnt == 0 || p.interpolated(b, cnt)) continue;
         const int o = p.pt[b];
         for (int j = 0; j < cnt; ++j) px[o + j] = xs[j0 + j];
     }
-    for (int i = p.m + threadIdx.x; i < m_pad; i += kThreads) px[i] = far;
+    for (int i = p.m + threadIdx.x; i < m_pad; i += (int)blockDim.x) px[i] = far;
 }
 
 // Sums at a panel's points -> Chebyshev coefficients, in place, one thread per
 // (panel, sum); sums are arrays r0 .. r0 + nq - 1 of STRIDE floats in pts.
 template <int STRIDE = kMaxPts>
 __device__ __forceinline__ void fast_coefficients(const FastTab& t, int nc, int r0, int nq) {
-    for (int it = threadIdx.x; it < nc * nq; it += kThreads) {
+    for (int it = threadIdx.x; it < nc * nq; it += (int)blockDim.x) {
         float* v = t.pts + (r0 + it / nc) * STRIDE + (it % nc) * kP;
         float a[kP];
 #pragma unroll
@@ -544,7 +549,7 @@ __device__ __forceinline__ void fast_point_sums(const FastTab& t, int m, int m_p
     const float* __restrict__ QG = t.pts + 2 * STRIDE;
     const float* __restrict__ QC = t.pts + 3 * STRIDE;
     const int grp = threadIdx.x / S, q = threadIdx.x % S;
-    for (int base = 0; base < m; base += R * kThreads / S) {
+    for (int base = 0; base < m; base += R * (int)blockDim.x / S) {
         const int r0 = base + R * grp;
         float2 xi[R], kg[R], gk[R], ks[R], kc[R], nk[R], gd[R], hs[R];
 #pragma unroll
@@ -552,6 +557,7 @@ __device__ __forceinline__ void fast_point_sums(const FastTab& t, int m, int m_p
             xi[r] = f2(X[min(r0 + r, m - 1)]);
             kg[r] = gk[r] = ks[r] = kc[r] = nk[r] = gd[r] = hs[r] = f2(0.0f);
         }
+#pragma unroll 2
         for (int cb = q * 4; cb < m_pad; cb += 4 * S) {
             const float4 x4 = *reinterpret_cast<const float4*>(X + cb);
             const float4 a4 = *reinterpret_cast<const float4*>(Q1 + cb);
@@ -767,7 +773,7 @@ __device__ __forceinline__ void fast_mixture_points(const FastTab& t, FastSh& sh
     const int grp = threadIdx.x / S, q = threadIdx.x % S;
     unsigned short* far_list = reinterpret_cast<unsigned short*>(t.pref);
     const float fs = kFineScale * src.up;
-    for (int base = 0; base < m; base += R * kThreads / S) {
+    for (int base = 0; base < m; base += R * (int)blockDim.x / S) {
         const int r0 = base + R * grp;
         float x[R];
         float2 x2[R], den2[R], num2[R];
@@ -816,7 +822,7 @@ __device__ __forceinline__ void fast_mixture_points(const FastTab& t, FastSh& sh
     }
     __syncthreads();
     // the far ones, a warp each (in any order: they are independent)
-    for (int k = threadIdx.x >> 5; k < sh.n_far; k += kWarps) {
+    for (int k = threadIdx.x >> 5; k < sh.n_far; k += (int)(blockDim.x >> 5)) {
         const int r = far_list[k];
         float den, num, e;
         mixture_far(scaled(t.pts[r]), t, src, n, mean, den, num, e);
@@ -835,7 +841,7 @@ __device__ __forceinline__ void fast_mixture_points(const FastTab& t, FastSh& sh
 // are summed one by one.
 __device__ __forceinline__ void fast_mixture_panels(const FastTab& t, const Panels& p, float unit) {
     const int lane = threadIdx.x & 31, q = lane & 15;
-    for (int base = 0; base < p.nc; base += kThreads / 16) {
+    for (int base = 0; base < p.nc; base += (int)blockDim.x / 16) {
         const int ci = base + threadIdx.x / 16;
         const bool on = ci < p.nc && q < kP;
         const int at = min(ci, p.nc - 1) * kP + min(q, kP - 1);

@@ -47,6 +47,24 @@ SVPF_HD inline bool fast_tick(int n, const svpf_config_t& c) {
            (!c.use_newton || c.use_full_newton);
 }
 
+// Whether the filters of a launch run on wide CTAs (512 threads, one per SM)
+// instead of two of 256 threads per SM.  A fast tick is a chain of phases whose
+// latencies more warps hide: alone on an SM, N = 512 takes 289 us narrow and
+// 216 wide, N = 320 251 and 200 (two narrow ones side by side 313 each), the
+// request round of 200 two-factor instruments (256 to 2048 particles) 2.92 ms
+// and 1.91.  Two narrow CTAs do more in all, so the line lies where the ticks
+// per SM add up to kWideLoad of the longest one.
+constexpr int kWideThreads = 512;
+constexpr double kWideLoad = 1.5;
+struct WideChoice {
+    double sum = 0.0, longest = 0.0;
+    int sms = 1;
+    bool ok = true;   // every filter goes through the fast sums or fits a one-row tile
+    WideChoice();
+    void add(int n, const svpf_config_t& c, int tile);
+    bool wide() const;
+};
+
 struct SingleArgs {
     svpf_config_t cfg;
     SVPFParams prm;
@@ -170,11 +188,11 @@ cudaError_t launch_single(const SingleArgs& a, int C, int tile, cudaStream_t s);
 cudaError_t launch_single_small(const SingleArgs& a, int C, int tile, cudaStream_t s);
 cudaError_t launch_single_large(const SingleArgs& a, int C, int tile, cudaStream_t s);
 cudaError_t launch_single_2f(const SingleArgs& a, int C, int tile, cudaStream_t s);
-cudaError_t launch_batch(const BatchArgs& a, size_t smem_bytes, int grid, cudaStream_t s);
-cudaError_t launch_batch_2f(const BatchArgs& a, size_t smem_bytes, int grid, cudaStream_t s);
+cudaError_t launch_batch(const BatchArgs& a, size_t smem_bytes, int grid, bool wide, cudaStream_t s);
+cudaError_t launch_batch_2f(const BatchArgs& a, size_t smem_bytes, int grid, bool wide, cudaStream_t s);
 cudaError_t launch_init(const InitArgs& a, cudaStream_t s);
-int batch_grid(size_t smem_bytes);
-int batch_grid_2f(size_t smem_bytes);
+int batch_grid(size_t smem_bytes, bool wide = false);
+int batch_grid_2f(size_t smem_bytes, bool wide = false);
 // Two-factor persistent kernel on clusters of kCluster2f (= 4) CTAs per filter.
 int batch_cluster_grid_2f(size_t smem_bytes);   // CTAs (a multiple of 4), 0 if it cannot run
 cudaError_t launch_batch_2f_cluster(const BatchArgs& a, size_t smem_bytes, int grid, cudaStream_t s);

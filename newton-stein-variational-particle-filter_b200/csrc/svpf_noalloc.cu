@@ -183,7 +183,7 @@ int svpf_batch_tick_noalloc(int n_filters, const int* d_n, const long long* d_of
     a.seed = seed;
     a.tape_stride = n_max;
     a.heun = any_heun != 0;
-    return launch_batch(a, smem, grid, stream) == cudaSuccess ? SVPF_OK : SVPF_ERR_CUDA;
+    return launch_batch(a, smem, grid, false, stream) == cudaSuccess ? SVPF_OK : SVPF_ERR_CUDA;
 }
 
 int svpf_noalloc_max_filters(void) { return SVPF_NOALLOC_MAX_FILTERS; }

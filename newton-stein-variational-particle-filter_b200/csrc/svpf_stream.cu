@@ -44,6 +44,7 @@ struct svpf_stream {
     std::vector<uint8_t> tiles;
     size_t smem1 = 0, smem2 = 0, smem2c = 0;
     int grid1 = 0, grid2 = 0, grid2c = 0;
+    int grid1w = 0, grid2w = 0;   // of wide CTAs (WideChoice)
     long long launches = 0;
     // device
     float* pool = nullptr;        // 4 arrays of pool_floats: h, h_prev, v, log_w
@@ -131,7 +132,7 @@ bool big_2f(const svpf_stream* s, int slot) {
 // stream, which then waits for both.  A kernel's CTAs take the SMs that another
 // kernel's tail frees instead of waiting for the whole kernel to end.
 int launch_round(svpf_stream* s, int c1, int c2, const int* d_req, const float* d_y, svpf_out_t* d_out,
-                 int c2c = 0) {
+                 int c2c = 0, bool wide1 = false, bool wide2 = false) {
     if (cudaMemsetAsync(s->d_queue, 0, 3 * sizeof(int), s->stream) != cudaSuccess) return SVPF_ERR_CUDA;
     if (cudaEventRecord(s->fork, s->stream) != cudaSuccess) return SVPF_ERR_CUDA;
     BatchArgs a = round_args(s);
@@ -157,7 +158,7 @@ int launch_round(svpf_stream* s, int c1, int c2, const int* d_req, const float* 
         a.req_y = d_y + c1 + c2c;
         a.out = d_out + c1 + c2c;
         if (cudaStreamWaitEvent(s->side[1], s->fork, 0) != cudaSuccess ||
-            launch_batch_2f(a, s->smem2, s->grid2, s->side[1]) != cudaSuccess ||
+            launch_batch_2f(a, s->smem2, wide2 ? s->grid2w : s->grid2, wide2, s->side[1]) != cudaSuccess ||
             cudaEventRecord(s->join[1], s->side[1]) != cudaSuccess)
             return SVPF_ERR_CUDA;
         joined[1] = true;
@@ -169,7 +170,7 @@ int launch_round(svpf_stream* s, int c1, int c2, const int* d_req, const float* 
         a.queue = s->d_queue;
         a.req_y = d_y;
         a.out = d_out;
-        if (launch_batch(a, s->smem1, s->grid1, s->stream) != cudaSuccess) return SVPF_ERR_CUDA;
+        if (launch_batch(a, s->smem1, wide1 ? s->grid1w : s->grid1, wide1, s->stream) != cudaSuccess) return SVPF_ERR_CUDA;
         ++s->launches;
     }
     for (int k = 0; k < 2; ++k)
@@ -236,11 +237,15 @@ svpf_stream_t* svpf_stream_create(int max_instruments, size_t hbm_budget_bytes, 
         svpf_config_init(&any, 1, SVPF_DEFAULT_NU);
         s->smem1 = tick_smem_bytes_batch(n_max, any, false);
         s->smem2 = tick_smem_bytes_2f(n_max, 1);
-        if (s->smem1 <= max_dyn_smem()) s->grid1 = batch_grid(s->smem1);
+        if (s->smem1 <= max_dyn_smem()) {
+            s->grid1 = batch_grid(s->smem1);
+            s->grid1w = batch_grid(s->smem1, true);
+        }
         if (s->smem2 <= max_dyn_smem()) {
             const size_t fast = tick_smem_bytes_2f_fast(n_max);
             if (fast <= max_dyn_smem()) s->smem2 = std::max(s->smem2, fast);
             s->grid2 = batch_grid_2f(s->smem2);
+            s->grid2w = batch_grid_2f(s->smem2, true);
         }
         s->smem2c = tick_smem_bytes_2f(n_max, kClusterMembers2f);
         if (n_max >= kClusterMinN && s->smem2c <= max_dyn_smem()) s->grid2c = batch_cluster_grid_2f(s->smem2c);
@@ -424,18 +429,22 @@ int svpf_stream_process(svpf_stream_t* s, int count, const int* slots, const flo
             return tick_cost(s->ns[slots[a]], s->cfgs[slots[a]]) > tick_cost(s->ns[slots[b]], s->cfgs[slots[b]]);
         });
         int c1 = 0, c2c = 0;
+        WideChoice w1, w2;
         for (size_t q = 0; q < idx.size(); ++q) {
             s->h_req[q] = slots[idx[q]];
             s->h_y[q] = y[idx[q]];
             const int gq = group(idx[q]);
             if (gq == 0) ++c1;
             if (gq == 1) ++c2c;
+            const int slot = slots[idx[q]];
+            if (gq != 1) (gq == 0 ? w1 : w2).add(s->ns[slot], s->cfgs[slot], s->tiles[slot]);
         }
         const int m = (int)idx.size();
         if (cudaMemcpyAsync(s->d_req, s->h_req, m * sizeof(int), cudaMemcpyHostToDevice, s->stream) != cudaSuccess ||
             cudaMemcpyAsync(s->d_y, s->h_y, m * sizeof(float), cudaMemcpyHostToDevice, s->stream) != cudaSuccess)
             return SVPF_ERR_CUDA;
-        const int rc = launch_round(s, c1, m - c1, s->d_req, s->d_y, s->d_out, c2c);
+        const int rc = launch_round(s, c1, m - c1, s->d_req, s->d_y, s->d_out, c2c, w1.wide() && s->grid1w > 0,
+                                    w2.wide() && s->grid2w > 0);
         if (rc != SVPF_OK) return rc;
         if (cudaMemcpyAsync(s->h_out, s->d_out, m * sizeof(svpf_out_t), cudaMemcpyDeviceToHost, s->stream) !=
                 cudaSuccess ||

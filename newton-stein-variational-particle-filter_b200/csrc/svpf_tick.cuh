@@ -51,10 +51,11 @@ __device__ __forceinline__ void grad_dispatch(bool student, const Smem& sm, int 
 }
 
 // KSD of the last iteration: block sum, then member partials into rank 0.
+template <int NT = kThreads>
 __device__ __forceinline__ void ksd_publish(float ksd_thread, Plan& pl, const Team& team) {
     float v[1] = {ksd_thread};
     const int op[1] = {0};
-    block_reduce<1>(v, op, pl);
+    block_reduce<1, NT>(v, op, pl);
     if (threadIdx.x == 0) team.at(pl.ksd_slot, 0)[team.rank] = v[0];
 }
 
@@ -135,7 +136,7 @@ __device__ inline bool fast_sources(FastWork& w, const Plan& pl, int n, FastSh& 
         fast_points(w.b, w.src.up, t, p, t.src_x, pad, kMuPad);
         auto none = [](int) { return 0.0f; };
         fast_weights<false, false, false>(w.b, w.src.up, t, p, t.src_w, nullptr, nullptr, none, none);
-        for (int i = p.m + threadIdx.x; i < pad; i += kThreads) t.src_w[i] = 0.0f;
+        for (int i = p.m + threadIdx.x; i < pad; i += blockDim.x) t.src_w[i] = 0.0f;
         __syncthreads();
         return true;
     }
@@ -151,7 +152,7 @@ template <bool PROD>
 __device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_config_t& cfg, const SVPFParams& prm,
                                const FilterIO& io, const Noise& nz, int kn, float beta, float bf, bool last,
                                FastSh& sh, float& ksd) {
-    const int tid = threadIdx.x, n = io.n;
+    const int tid = threadIdx.x, nt = blockDim.x, n = io.n;
     const FastTab& t = w.tab;
     fast_bin([&](int i) { return w.a[i]; }, n, kFineScale, w.b, w.pidx, t, sh);
     const Panels p = fast_panels(3, t.pt, t.comp, kMaxComp, kMaxPts, false, t, sh);
@@ -170,7 +171,7 @@ __device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_con
     const float inv_s2 = 1.0f / (pl.sz_eff * pl.sz_eff);
     const float nu = cfg.nu;
     const float y2 = pl.y_t * pl.y_t;
-    for (int base = 0; base < n; base += kThreads) {
+    for (int base = 0; base < n; base += nt) {
         const int s = base + tid;
         const bool on = s < n;
         const float x = w.b[min(s, n - 1)];
@@ -223,7 +224,7 @@ __device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_con
     __syncthreads();
     const int m = p.m, m_pad = round_up(m, 32);
     fast_points(w.b, 1.0f, t, p, t.pts, m_pad, kHPad);
-    for (int i = m + tid; i < m_pad; i += kThreads)
+    for (int i = m + tid; i < m_pad; i += nt)
         t.pts[kMaxPts + i] = t.pts[2 * kMaxPts + i] = t.pts[3 * kMaxPts + i] = 0.0f;
     auto gv = [&](int j) { return w.a[j]; };
     auto cv = [&](int j) { return w.c[j]; };
@@ -251,7 +252,7 @@ __device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_con
     const float inv_bw = pl.inv_bw, inv_bw2 = pl.inv_bw2, inv_n = 1.0f / (float)n;
     const float es = pl.eps_step * bf, rr = cfg.rmsprop_rho;
     ksd = 0.0f;
-    for (int s = tid; s < n; s += kThreads) {
+    for (int s = tid; s < n; s += nt) {
         const float x = w.b[s];
         const int i = w.pidx[s];
         const float v0 = io.v[i];
@@ -313,8 +314,8 @@ __device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_con
 // FAST: the Stein iterations go through the fast sums (one CTA, Gaussian state
 // noise, vanilla or full-Newton transport, no Heun step, dynamic shared memory
 // of fast_smem_floats); a tick whose particles do not fit them finishes with
-// the <R, S> sweeps.
-template <int R, int S, bool SCAN = false, bool PROD = false, int U = 0, bool FAST = false>
+// the <R, S> sweeps.  NT: threads of the CTA (no Heun step above kThreads).
+template <int R, int S, bool SCAN = false, bool PROD = false, int U = 0, bool FAST = false, int NT = kThreads>
 __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_ctl_t& ctl, float y_t,
                          float y_prev, const FilterIO& io, const Noise& nz, const Smem& sm, Plan& pl,
                          const Team& team, svpf_out_t& out, FastSh* fsh = nullptr) {
@@ -336,10 +337,10 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
     }
     // pads: particle columns [n, np) and prior slots [n, m_len)
     auto pads = [&]() {
-        for (int i = n + tid; i < sm.np; i += kThreads) {
+        for (int i = n + tid; i < sm.np; i += NT) {
             sm.h[0][i] = kHPad; sm.h[1][i] = kHPad; sm.g[i] = 0.0f; sm.c[i] = 0.0f;
         }
-        for (int i = n + tid; i < sm.m_len; i += kThreads) sm.mu[i] = kMuPad;
+        for (int i = n + tid; i < sm.m_len; i += NT) sm.mu[i] = kMuPad;
     };
     if constexpr (!FAST) pads();
     __syncthreads();
@@ -355,7 +356,7 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
         const float nm_pres = (1.0f - gsn) * hbar + gsn * gmean;
         const float ly2 = logf(y_t * y_t + 1e-10f);
         const float mimp = fmaxf(ly2 + pl.off, -5.0f);
-        for (int i = tid; i < n; i += kThreads) {
+        for (int i = tid; i < n; i += NT) {
             const float hi = io.h[i];
             const float hpi = io.h_prev[i];
             float z;
@@ -409,10 +410,10 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
     }
     if constexpr (FAST) {
         const int op[5] = {0, 0, 2, 1, 0};
-        block_reduce<5>(st, op, pl);
+        block_reduce<5, NT>(st, op, pl);
     } else {
         const int op[4] = {0, 0, 2, 1};
-        block_reduce<4>(st, op, pl);
+        block_reduce<4, NT>(st, op, pl);
     }
     // ---- bandwidth (svpf_fused_bandwidth_kernel, svpf_opt_kernels.cu:1159-1235)
     if (tid == 0) {
@@ -450,7 +451,7 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
     //      means (mu - mu_center) * prior_scale (order preserving)
     const bool student = PROD ? false : cfg.use_student_t_state != 0;
     if (pl.budget > 0) {
-        for (int i = tid; i < n; i += kThreads) {
+        for (int i = tid; i < n; i += NT) {
             sm.h[0][i] = (sm.h[0][i] - pl.center) * pl.inv_bw;
             if constexpr (FAST) sm.g[i] = (sm.g[i] - pl.mu_center) * pl.prior_scale;
             else if (!student) sm.mu[i] = (sm.mu[i] - pl.mu_center) * pl.prior_scale;
@@ -458,14 +459,14 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
     }
     // ---- own rows' RMSProp state (the fast iterations keep it in global memory)
     if constexpr (!FAST) {
-        for (int li = tid; li < sm.row1 - sm.row0; li += kThreads) sm.v[li] = io.v[sm.row0 + li];
+        for (int li = tid; li < sm.row1 - sm.row0; li += NT) sm.v[li] = io.v[sm.row0 + li];
     }
     // ---- SVLD normals of own rows for the first Stein iterations, drawn in
     //      parallel (same draws, in the same slots, as the per-row epilogue takes)
     if (sm.pre != nullptr && pl.temp > 1e-6f && (PROD || !cfg.use_heun)) {
         const int nloc = sm.row1 - sm.row0;
         const int iters = min(pl.budget, kPreIters);
-        for (int k = tid; k < iters * nloc; k += kThreads) {
+        for (int k = tid; k < iters * nloc; k += NT) {
             const int it = k / nloc, li = k - it * nloc;
             sm.pre[it * sm.Lp + li] = nz.normal(sm.row0 + li, pl.kn_pred + it);
         }
@@ -486,7 +487,7 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
                 float kt;
                 fits = fast_iteration<PROD>(fw, pl, cfg, prm, io, nz, kn, beta, sqrtf(beta), it0 == budget - 1, *fsh, kt);
                 if (!fits) break;
-                if (it0 == budget - 1) ksd_publish(kt, pl, team);
+                if (it0 == budget - 1) ksd_publish<NT>(kt, pl, team);
                 float* x = fw.c;
                 fw.c = fw.a;
                 fw.a = x;
@@ -498,10 +499,10 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
                 __syncthreads();
                 direct = true;
                 if (fw.a != sm.h[0])
-                    for (int i = tid; i < n; i += kThreads) sm.h[0][i] = fw.a[i];
+                    for (int i = tid; i < n; i += NT) sm.h[0][i] = fw.a[i];
                 __syncthreads();
                 pads();
-                for (int i = tid; i < n; i += kThreads) {
+                for (int i = tid; i < n; i += NT) {
                     sm.mu[i] = (prior_mean(io.h[i], pl, prm, y_prev) - pl.mu_center) * pl.prior_scale;
                     sm.v[i] = io.v[i];
                 }
@@ -510,6 +511,7 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
             }
         }
     }
+    const bool sweeps = NT == kThreads || tid < kThreads;   // a larger CTA sweeps with its first threads
     for (int it = it0; it < budget; ++it) {
         const int ai = stage_of(pl, it);
         const float beta = pl.beta[ai];
@@ -517,22 +519,24 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
         const bool last = it == budget - 1;
         if (PROD || !cfg.use_heun) {
             const float* pre = (sm.pre != nullptr && it < kPreIters) ? sm.pre + it * sm.Lp : nullptr;
-            float kt;
+            float kt = 0.0f;
             if constexpr (PROD) {
-                grad_pass<R, S, false, SCAN, U>(sm, cur, pl, cfg, beta, io.lw, team);
+                if (sweeps) grad_pass<R, S, false, SCAN, U>(sm, cur, pl, cfg, beta, io.lw, team);
                 team.sync();
-                kt = last ? stein_rows<R, S, 2, true, kTransport, U>(sm, cur, pl, cfg, bf, nz, kn, team, nullptr, pre)
+                if (sweeps)
+                    kt = last ? stein_rows<R, S, 2, true, kTransport, U>(sm, cur, pl, cfg, bf, nz, kn, team, nullptr, pre)
                           : stein_rows<R, S, 2, false, kTransport, U>(sm, cur, pl, cfg, bf, nz, kn, team, nullptr, pre);
             } else {
-                grad_dispatch<R, S, SCAN>(student, sm, cur, pl, cfg, beta, io.lw, team);
+                if (sweeps) grad_dispatch<R, S, SCAN>(student, sm, cur, pl, cfg, beta, io.lw, team);
                 team.sync();
-                kt = stein_dispatch<R, S, kTransport>(pl.transport, last, sm, cur, pl, cfg, bf, nz, kn, team,
+                if (sweeps)
+                    kt = stein_dispatch<R, S, kTransport>(pl.transport, last, sm, cur, pl, cfg, bf, nz, kn, team,
                                                       nullptr, pre);
             }
-            if (last) ksd_publish(kt, pl, team);
+            if (last) ksd_publish<NT>(kt, pl, team);
             team.sync();
             cur ^= 1;
-        } else if constexpr (!PROD) {
+        } else if constexpr (!PROD && NT == kThreads) {
             // Heun predictor-corrector (svpf_optimized_graph.cu:1147-1232,
             // kernels svpf_opt_kernels.cu:1293-1566)
             const int nloc = sm.row1 - sm.row0;
@@ -541,7 +545,7 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
             team.sync();
             stein_dispatch<R, S, kPhiOnly>(pl.transport, false, sm, cur, pl, cfg, bf, nz, kn, team, sm.phi0);
             __syncthreads();
-            for (int li = tid; li < nloc; li += kThreads) {
+            for (int li = tid; li < nloc; li += NT) {
                 const int i = sm.row0 + li;
                 const float h0 = fmaf(sm.h[cur][i], pl.bw, pl.center);
                 const float hpred = clamp_h(h0 + es * sm.phi0[li] * rsqrtf(sm.v[li] + cfg.rmsprop_eps));
@@ -555,10 +559,10 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
             if (last) {
                 // KSD at the start point with the gradient at the predicted point
                 const float kt = stein_dispatch<R, S, kKsdOnly>(0, true, sm, cur, pl, cfg, bf, nz, kn, team);
-                ksd_publish(kt, pl, team);
+                ksd_publish<NT>(kt, pl, team);
             }
             team.sync();   // all members done reading the predicted positions
-            for (int li = tid; li < nloc; li += kThreads) {
+            for (int li = tid; li < nloc; li += NT) {
                 const int i = sm.row0 + li;
                 const float pa = 0.5f * (sm.phi0[li] + sm.phi1[li]);
                 const float vn = cfg.rmsprop_rho * sm.v[li] + (1.0f - cfg.rmsprop_rho) * pa * pa;
@@ -578,7 +582,7 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
 
     // own rows' RMSProp state back to global memory
     if (direct) {
-        for (int li = tid; li < sm.row1 - sm.row0; li += kThreads) io.v[sm.row0 + li] = sm.v[li];
+        for (int li = tid; li < sm.row1 - sm.row0; li += NT) io.v[sm.row0 + li] = sm.v[li];
     }
     if (team.rank != 0) return;
 
@@ -597,14 +601,14 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
     if constexpr (FAST)
         if (!direct) hf = fw.a;
     if (budget > 0) {
-        for (int i = tid; i < n; i += kThreads) hf[i] = fmaf(hf[i], pl.bw, pl.center);
+        for (int i = tid; i < n; i += NT) hf[i] = fmaf(hf[i], pl.bw, pl.center);
         __syncthreads();
     }
     // ---- partial rejuvenation (svpf_opt_kernels.cu:1248-1275)
     if (pl.rejuv) {
         const int ku = pl.uses_uniform_predict;
         const float b = cfg.rejuv_blend;
-        for (int i = tid; i < n; i += kThreads) {
+        for (int i = tid; i < n; i += NT) {
             const float u = nz.uniform(i, ku);
             if (u < cfg.rejuv_prob) {
                 const float zz = nz.normal(i, kn);
@@ -616,23 +620,23 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
 
     // ---- outputs (svpf_fused_outputs_kernel, svpf_opt_kernels.cu:1109-1153)
     float mx[1] = {-1e10f};
-    for (int i = tid; i < n; i += kThreads) mx[0] = fmaxf(mx[0], io.lw[i]);
+    for (int i = tid; i < n; i += NT) mx[0] = fmaxf(mx[0], io.lw[i]);
     {
         const int op[1] = {1};
-        block_reduce<1>(mx, op, pl);
+        block_reduce<1, NT>(mx, op, pl);
     }
     float acc[3] = {0.0f, 0.0f, 0.0f};
-    for (int i = tid; i < n; i += kThreads) {
+    for (int i = tid; i < n; i += NT) {
         acc[0] += ex2_approx((io.lw[i] - mx[0]) * kLog2e);
         acc[1] += expf(fminf(hf[i] * 0.5f, 20.0f));
         acc[2] += hf[i];
     }
     {
         const int op[3] = {0, 0, 0};
-        block_reduce<3>(acc, op, pl);
+        block_reduce<3, NT>(acc, op, pl);
     }
     // write back positions: h_prev <- positions at tick start, h <- final
-    for (int i = tid; i < n; i += kThreads) {
+    for (int i = tid; i < n; i += NT) {
         io.h_prev[i] = io.h[i];
         io.h[i] = hf[i];
     }

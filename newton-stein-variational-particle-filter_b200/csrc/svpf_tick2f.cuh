@@ -79,7 +79,7 @@ __device__ inline void grad_pass_2f(const Smem2& sm, int cur, const Plan& pl, co
     const float half_np1 = 0.5f * (nu + 1.0f);
     const float* xf = sm.f[0].h[cur];
     const float* xs = sm.f[1].h[cur];
-    for (int i = threadIdx.x; i < n; i += kThreads) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const float hf = xf[i];
         const float hs = xs[i];
         const float hc = mu + hf + hs;
@@ -136,7 +136,7 @@ __device__ inline Smem2 carve_2f_fast(float* base, int n, FastWork2& w) {
 // step whose particles do not fit the tables sweeps over the pairs.
 __device__ inline void fast_transport_2f(const Smem& f, float* __restrict__ v, const FastWork2& w, const FactorPlan& fp,
                                          const svpf_config_t& cfg, float beta, const Noise& nz, int kn, FastSh& sh) {
-    const int tid = threadIdx.x, n = f.n;
+    const int tid = threadIdx.x, nt = blockDim.x, n = f.n;
     const FastTab& t = w.tab;
     float* x = f.h[0];
     const float* g = f.g;
@@ -145,9 +145,9 @@ __device__ inline void fast_transport_2f(const Smem& f, float* __restrict__ v, c
     const float inv_n = 1.0f / (float)n, rr = cfg.rmsprop_rho;
     const float es = fp.eps_step * beta;
     // the row's new position from its sums
-    auto move = [&](int i, float kg, float gk) {
+    auto move = [&](int i, float v0, float kg, float gk) {
         const float phi = (kg + sign * 2.0f * ib * gk) * inv_n;
-        const float vn = rr * v[i] + (1.0f - rr) * phi * phi;
+        const float vn = rr * v0 + (1.0f - rr) * phi * phi;
         v[i] = vn;
         const float drift = es * phi * rsqrtf(vn + cfg.rmsprop_eps);
         float diff = 0.0f;
@@ -157,7 +157,7 @@ __device__ inline void fast_transport_2f(const Smem& f, float* __restrict__ v, c
     fast_bin([&](int i) { return (x[i] - cen) * ib; }, n, kFineScale, w.xs, w.pidx, t, sh);
     const Panels p = fast_panels(3, t.pt, t.comp, kFineBins / kFine, kMaxPts2f, false, t, sh);
     if (sh.over) {
-        for (int i = tid; i < n; i += kThreads) {
+        for (int i = tid; i < n; i += nt) {
             const float xi = x[i] * ib;
             float kg = 0.0f, gk = 0.0f;
             for (int j = 0; j < n; ++j) {
@@ -166,16 +166,16 @@ __device__ inline void fast_transport_2f(const Smem& f, float* __restrict__ v, c
                 kg = fmaf(K, g[j], kg);
                 gk = fmaf(u, K * K, gk);
             }
-            w.xs[i] = move(i, kg, gk);
+            w.xs[i] = move(i, v[i], kg, gk);
         }
         __syncthreads();
-        for (int i = tid; i < n; i += kThreads) x[i] = w.xs[i];
+        for (int i = tid; i < n; i += nt) x[i] = w.xs[i];
         __syncthreads();
         return;
     }
     const int m_pad = round_up(p.m, 32);
     fast_points(w.xs, 1.0f, t, p, t.pts, m_pad, kHPad);
-    for (int i = p.m + tid; i < m_pad; i += kThreads) t.pts[kMaxPts2f + i] = t.pts[2 * kMaxPts2f + i] = 0.0f;
+    for (int i = p.m + tid; i < m_pad; i += nt) t.pts[kMaxPts2f + i] = t.pts[2 * kMaxPts2f + i] = 0.0f;
     fast_weights<true, false, false>(w.xs, 1.0f, t, p, t.pts + kMaxPts2f, t.pts + 2 * kMaxPts2f, nullptr,
                                      [&](int j) { return g[w.pidx[j]]; }, [](int) { return 0.0f; });
     __syncthreads();
@@ -183,9 +183,17 @@ __device__ inline void fast_transport_2f(const Smem& f, float* __restrict__ v, c
     __syncthreads();
     fast_coefficients<kMaxPts2f>(t, p.nc, 3, 2);
     __syncthreads();
-    for (int s = tid; s < n; s += kThreads) {
+    // the next particle's moment is fetched while one is moved
+    int i_next = w.pidx[min(tid, n - 1)];
+    float v_next = v[i_next];
+    for (int s = tid; s < n; s += nt) {
         const float u = w.xs[s];
-        const int i = w.pidx[s];
+        const int i = i_next;
+        const float v0 = v_next;
+        if (s + nt < n) {
+            i_next = w.pidx[s + nt];
+            v_next = v[i_next];
+        }
         const int b = fine_bin(u) / kFine;
         const int j0 = t.fstart[kFine * b];
         const float* row = t.pts + 3 * kMaxPts2f + p.pt[b];
@@ -199,13 +207,13 @@ __device__ inline void fast_transport_2f(const Smem& f, float* __restrict__ v, c
             kg = row[s - j0];
             gk = row[kMaxPts2f + s - j0];
         }
-        x[i] = move(i, kg, gk);
+        x[i] = move(i, v0, kg, gk);
     }
     __syncthreads();
 }
 
 // FAST: the transports go through the fast sums (one CTA; sm from carve_2f_fast).
-template <int R, int S, bool FAST = false>
+template <int R, int S, bool FAST = false, int NT = kThreads>
 __device__ void run_tick_2f(const svpf_config_t& cfg, const SVPFParams& prm, svpf_ctl_t& ctl, float y_t,
                             float y_prev, const FilterIO& io, const Noise& nz, const Smem2& sm, Plan& pl,
                             const Team& team, svpf_out_t& out, const FastWork2* fw = nullptr, FastSh* fsh = nullptr) {
@@ -217,7 +225,7 @@ __device__ void run_tick_2f(const svpf_config_t& cfg, const SVPFParams& prm, svp
         pl.flag = 0;
         make_plan_2f(cfg, prm, ctl, y_t, y_prev, pl);
     }
-    for (int i = n + tid; i < np; i += kThreads) {
+    for (int i = n + tid; i < np; i += NT) {
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
             sm.f[k].h[0][i] = kHPadRaw;
@@ -237,7 +245,7 @@ __device__ void run_tick_2f(const svpf_config_t& cfg, const SVPFParams& prm, svp
         const float cmf = pl.fmean[0], cms = pl.fmean[1];
         const float nmf = (1.0f - gs) * cmf + gs * pl.gmean2[0];
         const float nms = (1.0f - gs) * cms + gs * pl.gmean2[1];
-        for (int i = tid; i < n; i += kThreads) {
+        for (int i = tid; i < n; i += NT) {
             const float hf0 = io.h[i], hs0 = io.h[n + i];
             sm.prev[0][i] = hf0;
             sm.prev[1][i] = hs0;
@@ -268,7 +276,7 @@ __device__ void run_tick_2f(const svpf_config_t& cfg, const SVPFParams& prm, svp
     }
     {
         const int op[4] = {0, 0, 0, 0};
-        block_reduce<4>(st, op, pl);
+        block_reduce<4, NT>(st, op, pl);
     }
     // ---- Silverman bandwidth per factor (svpf_bandwidth_two_factor_kernel, :256-318)
     if (tid == 0) {
@@ -290,7 +298,7 @@ __device__ void run_tick_2f(const svpf_config_t& cfg, const SVPFParams& prm, svp
     __syncthreads();
     // ---- own rows' RMSProp state (positions stay in log-volatility units)
     const int row0 = sm.f[0].row0, nloc = sm.f[0].row1 - row0;
-    for (int li = tid; !FAST && li < nloc; li += kThreads) {
+    for (int li = tid; !FAST && li < nloc; li += NT) {
         sm.f[0].v[li] = io.v[row0 + li];
         sm.f[1].v[li] = io.v[n + row0 + li];
     }
@@ -312,8 +320,10 @@ __device__ void run_tick_2f(const svpf_config_t& cfg, const SVPFParams& prm, svp
                 fast_transport_2f(sm.f[0], io.v, *fw, pl.fac[0], cfg, beta, nz, kn, *fsh);
                 fast_transport_2f(sm.f[1], io.v + n, *fw, pl.fac[1], cfg, beta, nz, kn + 1, *fsh);
             } else {
-                transport_pass<R, S, 0, false, kTransport>(sm.f[0], cur, pl.fac[0], cfg, beta, nz, kn, team);
-                transport_pass<R, S, 0, false, kTransport>(sm.f[1], cur, pl.fac[1], cfg, beta, nz, kn + 1, team);
+                if (NT == kThreads || tid < kThreads) {   // a larger CTA sweeps with its first threads
+                    transport_pass<R, S, 0, false, kTransport>(sm.f[0], cur, pl.fac[0], cfg, beta, nz, kn, team);
+                    transport_pass<R, S, 0, false, kTransport>(sm.f[1], cur, pl.fac[1], cfg, beta, nz, kn + 1, team);
+                }
                 team.sync();
                 cur ^= 1;
             }
@@ -321,7 +331,7 @@ __device__ void run_tick_2f(const svpf_config_t& cfg, const SVPFParams& prm, svp
         }
     }
 
-    for (int li = tid; !FAST && li < nloc; li += kThreads) {
+    for (int li = tid; !FAST && li < nloc; li += NT) {
         io.v[row0 + li] = sm.f[0].v[li];
         io.v[n + row0 + li] = sm.f[1].v[li];
     }
@@ -331,13 +341,13 @@ __device__ void run_tick_2f(const svpf_config_t& cfg, const SVPFParams& prm, svp
     const float* hf = sm.f[0].h[cur];
     const float* hs = sm.f[1].h[cur];
     float mx[1] = {-1e30f};
-    for (int i = tid; i < n; i += kThreads) mx[0] = fmaxf(mx[0], io.lw[i]);
+    for (int i = tid; i < n; i += NT) mx[0] = fmaxf(mx[0], io.lw[i]);
     {
         const int op[1] = {1};
-        block_reduce<1>(mx, op, pl);
+        block_reduce<1, NT>(mx, op, pl);
     }
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    for (int i = tid; i < n; i += kThreads) {
+    for (int i = tid; i < n; i += NT) {
         acc[0] += expf(io.lw[i] - mx[0]);
         acc[1] += hf[i];
         acc[2] += hs[i];
@@ -345,9 +355,9 @@ __device__ void run_tick_2f(const svpf_config_t& cfg, const SVPFParams& prm, svp
     }
     {
         const int op[4] = {0, 0, 0, 0};
-        block_reduce<4>(acc, op, pl);
+        block_reduce<4, NT>(acc, op, pl);
     }
-    for (int i = tid; i < n; i += kThreads) {
+    for (int i = tid; i < n; i += NT) {
         io.h_prev[i] = sm.prev[0][i];
         io.h_prev[n + i] = sm.prev[1][i];
         io.h[i] = hf[i];
