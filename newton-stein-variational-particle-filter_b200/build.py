@@ -23,7 +23,7 @@ BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libsvpf_b200.so")
 INCLUDE = os.path.join(ROOT, "include")
 
-SOURCES = ["svpf_kernels.cu", "svpf_single_small.cu", "svpf_single_large.cu", "svpf_single_2f.cu",
+SOURCES = ["svpf_kernels.cu", "svpf_single_small.cu", "svpf_single_large.cu", "svpf_single_2f.cu", "svpf_single_fast.cu",
            "svpf_batch_kernel.cu", "svpf_capi.cu", "svpf_batch.cu", "svpf_noalloc.cu", "svpf_grad.cu",
            "svpf_stream.cu", "svpf_v2.cu",
            "svpf_multiscale.cu", "svpf_estimator.cu", "svpf_calib.cu"]

@@ -330,7 +330,12 @@ void step_impl(SVPFState* s, float y_t, float y_prev, const SVPFParams* params,
         return;
     }
     const int tile = im->tile >= 0 ? im->tile : default_single_tile(s->n_particles, C);
-    cudaError_t e = tf ? launch_single_2f(a, C, tile, s->stream) : launch_single(a, C, tile, s->stream);
+    // a forced cluster size or tile is one of the sweeps
+    const bool fast = !tf && im->cluster == 0 && im->tile < 0 && s->n_particles >= kFastMinNSingle &&
+                      fast_tick(s->n_particles, a.cfg) && C > 1 &&
+                      tick_smem_bytes_single_fast(s->n_particles, C) <= max_dyn_smem();
+    cudaError_t e = tf ? launch_single_2f(a, C, tile, s->stream)
+                    : fast ? launch_single_fast(a, C, s->stream) : launch_single(a, C, tile, s->stream);
     if (e == cudaSuccess) e = wait_done(im, s->stream);
     if (e != cudaSuccess) {
         set_err(s, SVPF_ERR_CUDA);

@@ -32,8 +32,8 @@
 //    curvature of one Gaussian and a tilt that levels the panel's ends, before
 //    they are interpolated (numerator and denominator apart: both entire).
 //    Where the expansion has not converged -- a gap of many sigma between the
-//    prior means -- the panel's particles are summed one by one.  A point far outside the prior means gets its sums over all N
-//    means too, unless single means (kept exactly) dominate there.
+//    prior means -- and at points far outside the means, the sum goes over the
+//    means themselves that matter there, which stay sorted in global memory.
 //
 // A tick whose particles do not fit these tables (kFineBins bins, kMaxPts
 // points) finishes with the direct loops.
@@ -146,6 +146,7 @@ struct FastTab {
     float* src_w;
     unsigned short* fstart;   // [kFineBins + 1] first slot of each fine bin
     unsigned short* src_pt;   // [kFineBins / kFine + 1] first point of each panel of the prior means
+    unsigned short* src_slot; // the same for the sorted means themselves
     unsigned short* pt;       // transport panels: first points, [kFineBins / kFine]
     unsigned short* comp;     // [kFineBins / kFine]
     unsigned short* mpt;      // mixture panels: first points, [kFineBins]
@@ -162,7 +163,7 @@ struct FastSh {
 constexpr int kTabBasis = kP * kP + 16;
 constexpr int kTabPts = kPtRows * kMaxPts;
 constexpr int kTabPref = kMaxComp * kFine * kP;
-constexpr int kTabShorts = (kFineBins + 8) + (kFineBins / kFine + 8) + 2 * (kFineBins / kFine) + kFineBins +
+constexpr int kTabShorts = (kFineBins + 8) + 2 * (kFineBins / kFine + 8) + 2 * (kFineBins / kFine) + kFineBins +
                            2 * kMixComp;
 // binning counters and ranks take the points' space and the one behind it
 static_assert(kMixPts / 2 <= kTabPref, "the list of far points takes pref's space");
@@ -198,6 +199,8 @@ __device__ inline FastTab carve_fast(float* p, int np, bool mixture) {
     t.fstart = q;
     q += kFineBins + 8;
     t.src_pt = q;
+    q += kFineBins / kFine + 8;
+    t.src_slot = q;
     q += kFineBins / kFine + 8;
     t.pt = q;
     q += kFineBins / kFine;
@@ -512,12 +515,13 @@ __device__ __forceinline__ void fast_points(const float* __restrict__ xs, float 
     for (int i = p.m + threadIdx.x; i < m_pad; i += (int)blockDim.x) px[i] = far;
 }
 
-// Sums at a panel's points -> Chebyshev coefficients, in place, one thread per
+// Sums at the points of panels c0 .. c1 - 1 -> Chebyshev coefficients, in place, one thread per
 // (panel, sum); sums are arrays r0 .. r0 + nq - 1 of STRIDE floats in pts.
 template <int STRIDE = kMaxPts>
-__device__ __forceinline__ void fast_coefficients(const FastTab& t, int nc, int r0, int nq) {
+__device__ __forceinline__ void fast_coefficients(const FastTab& t, int c0, int c1, int r0, int nq) {
+    const int nc = c1 - c0;
     for (int it = threadIdx.x; it < nc * nq; it += (int)blockDim.x) {
-        float* v = t.pts + (r0 + it / nc) * STRIDE + (it % nc) * kP;
+        float* v = t.pts + (r0 + it / nc) * STRIDE + (c0 + it % nc) * kP;
         float a[kP];
 #pragma unroll
         for (int q = 0; q < kP; q += 4) *reinterpret_cast<float4*>(a + q) = *reinterpret_cast<const float4*>(v + q);
@@ -537,24 +541,62 @@ __device__ __forceinline__ void fast_coefficients(const FastTab& t, int nc, int 
     }
 }
 
+// The points a CTA sums at: all of them, or a cluster member's, those of the
+// panels its slots lie in (interpolated ones, then single points).
+struct PointRange {
+    int c0, c1;               // its interpolated panels
+    int nc, d0, count;        // points of interpolated panels, first single point, all
+    __device__ __forceinline__ int at(int k) const { return k < nc ? kP * c0 + k : d0 + (k - nc); }
+};
+__device__ __forceinline__ PointRange all_points(const Panels& p) { return PointRange{0, p.nc, kP * p.nc, kP * p.nc, p.m}; }
+__device__ inline PointRange member_points(const Panels& p, const float* __restrict__ xs, int s0, int s1,
+                                           const FastTab& t) {
+    PointRange r{0, 0, 0, 0, 0};
+    if (s0 >= s1) return r;
+    const int b0 = fine_bin(xs[s0]) >> p.sft, b1 = fine_bin(xs[s1 - 1]) >> p.sft;
+    auto before = [&](int b) {   // interpolated panels below b
+        int lo = 0, hi = p.nc;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (p.comp[mid] < b) lo = mid + 1; else hi = mid;
+        }
+        return lo;
+    };
+    r.c0 = before(b0);
+    r.c1 = before(b1 + 1);
+    r.nc = kP * (r.c1 - r.c0);
+    int d0 = 1 << 20, d1 = 0;
+    for (int b = b0 + (threadIdx.x & 31); b <= b1; b += 32) {
+        const int c = t.fstart[(b + 1) << p.sft] - t.fstart[b << p.sft];
+        if (c == 0 || p.interpolated(b, c)) continue;
+        d0 = min(d0, (int)p.pt[b]);
+        d1 = max(d1, (int)p.pt[b] + c);
+    }
+    d0 = __reduce_min_sync(0xffffffffu, d0);
+    d1 = __reduce_max_sync(0xffffffffu, d1);
+    r.d0 = d0;
+    r.count = r.nc + max(d1 - d0, 0);
+    return r;
+}
+
 // Transport sums at the points (arrays OUT.. of STRIDE floats in pts: sum K g, sum u K^2, then for
 // full Newton sum K, sum K c, sum K (3 - 4K), then for the KSD sum g u K^2 and
 // sum K^2 (3 - 4K)) over the points' weights.  Eight lanes share the columns of
 // two points: with 150 to 300 points that keeps every thread in work.
 template <bool FULL, bool KSD, int STRIDE = kMaxPts, int OUT = 4>
-__device__ __forceinline__ void fast_point_sums(const FastTab& t, int m, int m_pad) {
+__device__ __forceinline__ void fast_point_sums(const FastTab& t, const PointRange& own, int m_pad) {
     constexpr int S = 8, R = 2;
     const float* __restrict__ X = t.pts;
     const float* __restrict__ Q1 = t.pts + STRIDE;
     const float* __restrict__ QG = t.pts + 2 * STRIDE;
     const float* __restrict__ QC = t.pts + 3 * STRIDE;
     const int grp = threadIdx.x / S, q = threadIdx.x % S;
-    for (int base = 0; base < m; base += R * (int)blockDim.x / S) {
+    for (int base = 0; base < own.count; base += R * (int)blockDim.x / S) {
         const int r0 = base + R * grp;
         float2 xi[R], kg[R], gk[R], ks[R], kc[R], nk[R], gd[R], hs[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            xi[r] = f2(X[min(r0 + r, m - 1)]);
+            xi[r] = f2(X[own.at(min(r0 + r, own.count - 1))]);
             kg[r] = gk[r] = ks[r] = kc[r] = nk[r] = gd[r] = hs[r] = f2(0.0f);
         }
 #pragma unroll 2
@@ -602,7 +644,7 @@ __device__ __forceinline__ void fast_point_sums(const FastTab& t, int m, int m_p
                 if ((k >= 2 && k < 5 && !FULL) || (k >= 5 && !KSD)) continue;
 #pragma unroll
                 for (int o = S / 2; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-                if (q == 0 && r0 + r < m) t.pts[(OUT + k) * STRIDE + r0 + r] = v[k];
+                if (q == 0 && r0 + r < own.count) t.pts[(OUT + k) * STRIDE + own.at(r0 + r)] = v[k];
             }
         }
     }
@@ -668,37 +710,33 @@ __device__ __forceinline__ float fast_window(float x, const float* __restrict__ 
     return acc.x + acc.y;
 }
 
-// Mixture sums at x over all n prior means by one warp (every lane gets them):
-// den = sum w, num = sum w d, w = 2^-(d^2 - e), e the smallest d^2.
-// mean(k): the k-th scaled prior mean.
-template <class FM>
-__device__ __forceinline__ void mixture_exact(float x, int n, FM mean, float& den, float& num, float& e) {
-    const int lane = threadIdx.x & 31;
-    float mn = 3.0e38f;
-    for (int k = lane; k < n; k += 32) {
-        const float d = x - mean(k);
-        mn = fminf(mn, d * d);
-    }
-    mn = warp_min(mn);
-    float a = 0.0f, b = 0.0f;
-    for (int k = lane; k < n; k += 32) {
-        const float d = x - mean(k);
-        const float w = ex2_approx(mn - d * d);
-        a += w;
-        b = fmaf(w, d, b);
-    }
-    den = warp_sum(a);
-    num = warp_sum(b);
-    e = mn;
-}
-
 // The prior means' points: ns of them, panels of width kPanelW / up scaled units.
 struct Sources {
     int ns;
     float up;
     int near;          // a mean within this many panels of a point's own: the point is not far
     float far2;        // squared distance to which an interpolated panel's sum keeps its accuracy
+    const float* sorted;   // the means themselves by slot, in global memory
 };
+
+// Mixture sums at x over the prior means themselves, by one warp (every lane
+// gets them): den = sum w, num = sum w d, w = 2^-(d^2 - e), e about the
+// smallest d^2.  Means that weigh less than 2^-40 of the nearest are left out.
+__device__ __forceinline__ void mixture_exact(float x, const FastTab& t, const Sources& src, float e, float& den,
+                                              float& num) {
+    const int lane = threadIdx.x & 31;
+    const float fs = kFineScale * src.up, reach = sqrtf(e + 40.0f);
+    const int k0 = t.src_slot[fine_bin(x - reach, fs) / kFine], k1 = t.src_slot[fine_bin(x + reach, fs) / kFine + 1];
+    float a = 0.0f, b = 0.0f;
+    for (int k = k0 + lane; k < k1; k += 32) {
+        const float d = x - src.sorted[k];
+        const float w = ex2_approx(e - d * d);
+        a += w;
+        b = fmaf(w, d, b);
+    }
+    den = warp_sum(a);
+    num = warp_sum(b);
+}
 
 // Whether a point may be far from every mean: no mean in the panels around its
 // own, or these reach the first or last panel, whose outliers may lie anywhere
@@ -711,10 +749,9 @@ __device__ __forceinline__ bool mixture_is_far(float x, const FastTab& t, const 
 
 // Mixture sums at a point far from every mean, by one warp.  An interpolated
 // panel's sum is accurate relative to its largest term; single means must
-// outweigh it by 2^34, or all means are summed.
-template <class FM>
-__device__ __noinline__ void mixture_far(float x, const FastTab& t, const Sources& src, int n, FM mean, float& den,
-                                         float& num, float& e) {
+// outweigh it by 2^34, or the means themselves are summed.
+__device__ __forceinline__ void mixture_far(float x, const FastTab& t, const Sources& src, float& den, float& num,
+                                         float& e) {
     const int lane = threadIdx.x & 31;
     float ec = 3.0e38f, ed = 3.0e38f;   // nearest interpolated point, nearest single mean (weight exactly 1)
     for (int k = lane; k < src.ns; k += 32) {
@@ -726,7 +763,7 @@ __device__ __noinline__ void mixture_far(float x, const FastTab& t, const Source
     ed = warp_min(ed);
     e = fminf(ec, ed);
     if (e > src.far2 && ec < ed + 34.0f) {
-        mixture_exact(x, n, mean, den, num, e);
+        mixture_exact(x, t, src, e, den, num);
         return;
     }
     float a = 0.0f, b = 0.0f;
@@ -741,14 +778,12 @@ __device__ __noinline__ void mixture_far(float x, const FastTab& t, const Source
 }
 
 // Mixture sums at one point by one warp.
-template <class FM>
-__device__ __forceinline__ void mixture_warp(float x, const FastTab& t, const Sources& src, int n, FM mean, float& den,
-                                             float& num) {
+__device__ __forceinline__ void mixture_warp(float x, const FastTab& t, const Sources& src, float& den, float& num) {
     const int lane = threadIdx.x & 31;
     const float fs = kFineScale * src.up;
     if (mixture_is_far(x, t, src)) {
         float e;
-        mixture_far(x, t, src, n, mean, den, num, e);
+        mixture_far(x, t, src, den, num, e);
         return;
     }
     const int c0 = t.src_pt[fine_bin(x - kMixReach, fs) / kFine], c1 = t.src_pt[fine_bin(x + kMixReach, fs) / kFine + 1];
@@ -766,21 +801,21 @@ __device__ __forceinline__ void mixture_warp(float x, const FastTab& t, const So
 // Mixture sums at the points, [4][kMixPts] of pts: den, num, e (w = 2^-(d^2 - e);
 // e = 0 unless the point is far from every mean) over the prior means' points
 // within reach.  Eight lanes share the columns of two neighbouring points.
-template <class FX, class FM>
-__device__ __forceinline__ void fast_mixture_points(const FastTab& t, FastSh& sh, int m, const Sources& src, int n,
-                                                    FX scaled, FM mean) {
+template <class FX>
+__device__ __forceinline__ void fast_mixture_points(const FastTab& t, FastSh& sh, const PointRange& own,
+                                                    const Sources& src, FX scaled) {
     constexpr int S = 8, R = 2;
     const int grp = threadIdx.x / S, q = threadIdx.x % S;
     unsigned short* far_list = reinterpret_cast<unsigned short*>(t.pref);
     const float fs = kFineScale * src.up;
-    for (int base = 0; base < m; base += R * (int)blockDim.x / S) {
+    for (int base = 0; base < own.count; base += R * (int)blockDim.x / S) {
         const int r0 = base + R * grp;
         float x[R];
         float2 x2[R], den2[R], num2[R];
         bool far[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            x[r] = scaled(t.pts[min(r0 + r, m - 1)]);
+            x[r] = scaled(t.pts[own.at(min(r0 + r, own.count - 1))]);
             x2[r] = f2(x[r]);
             den2[r] = num2[r] = f2(0.0f);
             far[r] = mixture_is_far(x[r], t, src);
@@ -812,12 +847,13 @@ __device__ __forceinline__ void fast_mixture_points(const FastTab& t, FastSh& sh
                 den += __shfl_xor_sync(0xffffffffu, den, o);
                 num += __shfl_xor_sync(0xffffffffu, num, o);
             }
-            if (q == 0 && r0 + r < m) {
-                t.pts[kMixPts + r0 + r] = den;
-                t.pts[2 * kMixPts + r0 + r] = num;
-                t.pts[3 * kMixPts + r0 + r] = 0.0f;
+            if (q == 0 && r0 + r < own.count) {
+                const int at = own.at(r0 + r);
+                t.pts[kMixPts + at] = den;
+                t.pts[2 * kMixPts + at] = num;
+                t.pts[3 * kMixPts + at] = 0.0f;
+                if (far[r]) far_list[atomicAdd(&sh.n_far, 1)] = (unsigned short)at;
             }
-            if (q == 0 && r0 + r < m && far[r]) far_list[atomicAdd(&sh.n_far, 1)] = (unsigned short)(r0 + r);
         }
     }
     __syncthreads();
@@ -825,7 +861,7 @@ __device__ __forceinline__ void fast_mixture_points(const FastTab& t, FastSh& sh
     for (int k = threadIdx.x >> 5; k < sh.n_far; k += (int)(blockDim.x >> 5)) {
         const int r = far_list[k];
         float den, num, e;
-        mixture_far(scaled(t.pts[r]), t, src, n, mean, den, num, e);
+        mixture_far(scaled(t.pts[r]), t, src, den, num, e);
         if ((threadIdx.x & 31) == 0) {
             t.pts[kMixPts + r] = den;
             t.pts[2 * kMixPts + r] = num;
@@ -839,12 +875,12 @@ __device__ __forceinline__ void fast_mixture_points(const FastTab& t, FastSh& sh
 // last coefficients have not fallen to FP32 rounding (the sums change over
 // from one prior mean to another many sigma away) is marked: its particles
 // are summed one by one.
-__device__ __forceinline__ void fast_mixture_panels(const FastTab& t, const Panels& p, float unit) {
+__device__ __forceinline__ void fast_mixture_panels(const FastTab& t, const Panels& p, const PointRange& own, float unit) {
     const int lane = threadIdx.x & 31, q = lane & 15;
-    for (int base = 0; base < p.nc; base += (int)blockDim.x / 16) {
+    for (int base = own.c0; base < own.c1; base += (int)blockDim.x / 16) {
         const int ci = base + threadIdx.x / 16;
-        const bool on = ci < p.nc && q < kP;
-        const int at = min(ci, p.nc - 1) * kP + min(q, kP - 1);
+        const bool on = ci < own.c1 && q < kP;
+        const int at = min(ci, own.c1 - 1) * kP + min(q, kP - 1);
         const float den = t.pts[kMixPts + at], num = t.pts[2 * kMixPts + at], e = t.pts[3 * kMixPts + at];
         const float y = t.basis[kP * kP + min(q, kP - 1)] * unit / p.narrow;
         const float L = e - lg2_approx(den) - y * y;   // -log2 of the sum, less one Gaussian's curvature

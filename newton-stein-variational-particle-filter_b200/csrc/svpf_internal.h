@@ -65,6 +65,14 @@ struct WideChoice {
     bool wide() const;
 };
 
+// Single filters (one cluster of 16 CTAs) take the fast sums from this many
+// particles on.  Full-budget ticks on B200, fast sums against the sweeps, in
+// us: production settings N = 1100 207/215, 1500 217/257, 2048 234/319, 4096
+// 308/945, 8192 446/4043; no heat, 10 annealed steps of vanilla transport: 2048
+// 304/397, 8192 579/5121; sigma 0.15 and 16 steps: 1100 377/354, 1500 602/439
+// (some ticks do not fit the tables and do both), 2048 454/557, 8192 971/7751.
+constexpr int kFastMinNSingle = 2048;
+
 struct SingleArgs {
     svpf_config_t cfg;
     SVPFParams prm;
@@ -151,6 +159,8 @@ size_t tick_smem_bytes(int n, int C, bool heun);
 size_t tick_smem_bytes_batch(int n, const svpf_config_t& c, bool heun);
 // The single-filter kernel's: the tick's layout plus the pre-drawn SVLD normals.
 size_t tick_smem_bytes_single(int n, int C, bool heun);
+// The single-filter kernel's through the fast sums, on a cluster of C CTAs.
+size_t tick_smem_bytes_single_fast(int n, int C);
 size_t tick_smem_bytes_2f(int n, int C);
 size_t tick_smem_bytes_2f_fast(int n);
 // Largest dynamic shared memory a CTA may use on the current device.
@@ -185,6 +195,7 @@ int default_batch_tile(int n);
 int default_cluster(int n);
 
 cudaError_t launch_single(const SingleArgs& a, int C, int tile, cudaStream_t s);
+cudaError_t launch_single_fast(const SingleArgs& a, int C, cudaStream_t s);
 cudaError_t launch_single_small(const SingleArgs& a, int C, int tile, cudaStream_t s);
 cudaError_t launch_single_large(const SingleArgs& a, int C, int tile, cudaStream_t s);
 cudaError_t launch_single_2f(const SingleArgs& a, int C, int tile, cudaStream_t s);

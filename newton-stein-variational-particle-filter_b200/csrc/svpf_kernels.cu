@@ -77,6 +77,10 @@ size_t tick_smem_bytes_batch(int n, const svpf_config_t& c, bool heun) {
 size_t tick_smem_bytes_single(int n, int C, bool heun) {
     return (size_t)(smem_floats(n, C, heun) + pre_floats(n, C)) * sizeof(float);
 }
+size_t tick_smem_bytes_single_fast(int n, int C) {
+    const int sweeps = smem_floats(n, C, false), fast = fast_smem_floats(n, true);
+    return (size_t)(fast > sweeps ? fast : sweeps) * sizeof(float);
+}
 size_t tick_smem_bytes_2f_fast(int n) { return (size_t)fast_smem_floats_2f(n) * sizeof(float); }
 size_t tick_smem_bytes_2f(int n, int C) { return (size_t)smem_floats_2f(n, C) * sizeof(float); }
 

@@ -93,28 +93,51 @@ __device__ __forceinline__ float prior_mean(float h, const Plan& pl, const SVPFP
     return pl.mu_eff + prm.rho * (h - pl.mu_eff) + (lev != 0.0f ? lev / (expf(h * 0.5f) + 1e-8f) : 0.0f);
 }
 
-// Workspace of the fast tick (one CTA): particle-order and slot-order arrays
-// of n floats, the slots' particles, the tables (svpf_fast.cuh).
+// Workspace of the fast tick: arrays of n floats, the slots' particles, the
+// tables (svpf_fast.cuh).  One CTA keeps three arrays: g takes the positions'
+// place once they are binned, the next positions the curvatures'.  The members
+// of a cluster each have all particles, write one another's arrays and keep
+// four.
 struct FastWork {
-    float* a;                 // positions in particle order; g by slot once they are binned
-    float* b;                 // positions by slot
-    float* c;                 // curvature by slot; then the next positions in particle order
+    float* x;                 // positions, by particle
+    float* xs;                // positions, by slot
+    float* g;                 // transport score, by slot
+    float* c;                 // curvature, by slot
+    float* xn;                // next positions, by particle
+    float* means;             // scaled prior means, until the sources are built
     unsigned short* pidx;     // particle of a slot
     FastTab tab;
     Sources src;              // the prior means
     int sft;                  // fine bins of a mixture panel, log2
 };
 
-// Floats of dynamic shared memory of a fast tick.
-__host__ __device__ inline int fast_smem_floats(int n) {
+// Floats of dynamic shared memory of a fast tick, on one CTA or a cluster.
+__host__ __device__ inline int fast_smem_floats(int n, bool cluster = false) {
     const int np = round_up(n, 64);
-    return 3 * np + np / 2 + fast_table_floats(np, true);
+    return (cluster ? 4 : 3) * np + np / 2 + fast_table_floats(np, true);
+}
+__device__ inline void carve_fast_work(FastWork& w, const Smem& sm, bool cluster) {
+    w.x = sm.h[0];
+    w.xs = sm.h[1];
+    w.means = sm.g;
+    float* rest = cluster ? sm.mu : sm.c;   // sm: h, h, g, c, mu, ... of np floats each
+    if (cluster) {
+        w.g = sm.g;
+        w.c = sm.c;
+        w.xn = w.x;
+    } else {
+        w.g = w.x;
+        w.c = w.xn = sm.g;
+    }
+    w.pidx = reinterpret_cast<unsigned short*>(rest);
+    w.tab = carve_fast(rest + sm.np / 2, sm.np, true);
 }
 
-// The scaled prior means (w.c) as points, once per tick, in panels of 0.75
+// The scaled prior means as points, once per tick, in panels of 0.75
 // scaled units, or of 1.5 where that many do not fit.  False: they do not fit,
 // or one fine bin is too wide for the mixture.
-__device__ inline bool fast_sources(FastWork& w, const Plan& pl, int n, FastSh& sh) {
+__device__ inline bool fast_sources(FastWork& w, const Plan& pl, const FilterIO& io, FastSh& sh) {
+    const int n = io.n;
     const float unit = pl.bw * pl.prior_scale;   // scaled units per bandwidth
     w.sft = 3;
     while (w.sft > 0 && kFineW * unit * (float)(1 << w.sft) > kMixPanelMax) --w.sft;
@@ -124,7 +147,7 @@ __device__ inline bool fast_sources(FastWork& w, const Plan& pl, int n, FastSh& 
         w.src.up = wide ? 0.5f : 1.0f;
         w.src.near = wide ? 0 : 3;
         w.src.far2 = wide ? 5.0625f : 20.25f;
-        fast_bin([&](int i) { return w.c[i]; }, n, kFineScale * w.src.up, w.b, w.pidx, t, sh);
+        fast_bin([&](int i) { return w.means[i]; }, n, kFineScale * w.src.up, w.xs, w.pidx, t, sh);
         const Panels p = fast_panels(3, t.src_pt, t.comp, kFineBins / kFine, kMaxSrc, true, t, sh);
         if (sh.over) {
             __syncthreads();   // everyone has read it
@@ -132,10 +155,15 @@ __device__ inline bool fast_sources(FastWork& w, const Plan& pl, int n, FastSh& 
         }
         w.src.ns = p.m;
         if (threadIdx.x == 0) t.src_pt[kFineBins / kFine] = (unsigned short)p.m;
+        // The sorted means stay in h_prev, which has been read and is rewritten at
+        // the tick's end (the members of a cluster write the same values).
+        for (int k = threadIdx.x; k < n; k += blockDim.x) io.h_prev[k] = w.xs[k];
+        for (int b = threadIdx.x; b <= kFineBins / kFine; b += blockDim.x) t.src_slot[b] = t.fstart[kFine * b];
+        w.src.sorted = io.h_prev;
         const int pad = min(round_up(p.m, 4), kMaxSrc);
-        fast_points(w.b, w.src.up, t, p, t.src_x, pad, kMuPad);
+        fast_points(w.xs, w.src.up, t, p, t.src_x, pad, kMuPad);
         auto none = [](int) { return 0.0f; };
-        fast_weights<false, false, false>(w.b, w.src.up, t, p, t.src_w, nullptr, nullptr, none, none);
+        fast_weights<false, false, false>(w.xs, w.src.up, t, p, t.src_w, nullptr, nullptr, none, none);
         for (int i = p.m + threadIdx.x; i < pad; i += blockDim.x) t.src_w[i] = 0.0f;
         __syncthreads();
         return true;
@@ -143,38 +171,45 @@ __device__ inline bool fast_sources(FastWork& w, const Plan& pl, int n, FastSh& 
     return false;
 }
 
-// One Stein iteration of a filter on one CTA through the fast sums
-// (svpf_fast.cuh): gradient pass (svpf_opt_kernels.cu:354-521), vanilla or
+// One Stein iteration of a filter through the fast sums (svpf_fast.cuh): gradient pass (svpf_opt_kernels.cu:354-521), vanilla or
 // full-Newton transport (:527-1103) as grad_pass and transport_pass take it.
-// Positions: w.a before, w.c after (w.a untouched when it returns false: the
+// Positions: w.x before, w.xn after (w.x untouched when it returns false: the
 // particles do not fit the tables).  ksd: this thread's KSD terms.
+// In a cluster every member bins all particles (a copy of the same work: it
+// costs less than exchanging the order) and sums at the points and moves the
+// particles of its own slots; scores, curvatures and new positions go to every
+// member through distributed shared memory, one cluster barrier after each.
 template <bool PROD>
-__device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_config_t& cfg, const SVPFParams& prm,
+__device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_config_t& cfg,
                                const FilterIO& io, const Noise& nz, int kn, float beta, float bf, bool last,
-                               FastSh& sh, float& ksd) {
+                               const Team& team, FastSh& sh, float& ksd) {
     const int tid = threadIdx.x, nt = blockDim.x, n = io.n;
     const FastTab& t = w.tab;
-    fast_bin([&](int i) { return w.a[i]; }, n, kFineScale, w.b, w.pidx, t, sh);
+    fast_bin([&](int i) { return w.x[i]; }, n, kFineScale, w.xs, w.pidx, t, sh);
     const Panels p = fast_panels(3, t.pt, t.comp, kMaxComp, kMaxPts, false, t, sh);
     // the mixture's panels: the same ones unless they are too many sigma wide
     const Panels q = w.sft == 3 ? p : fast_panels(w.sft, t.mpt, t.mcomp, kMixComp, kMixPts, false, t, sh);
     if (sh.over) return false;
-    fast_points(w.b, 1.0f, t, q, t.pts, q.m, kHPad);
+    const int per = (n + team.size - 1) / team.size;
+    const int s0 = min(team.rank * per, n), s1 = min(s0 + per, n);   // own slots
+    const bool alone = team.size == 1;
+    const PointRange own = alone ? all_points(p) : member_points(p, w.xs, s0, s1, t);
+    const PointRange mix = alone ? all_points(q) : w.sft == 3 ? own : member_points(q, w.xs, s0, s1, t);
+    fast_points(w.xs, 1.0f, t, q, t.pts, q.m, kHPad);
     __syncthreads();
     auto scaled = [&](float x) { return (fmaf(x, pl.bw, pl.center) - pl.mu_center) * pl.prior_scale; };
-    auto mean = [&](int k) { return (prior_mean(io.h[k], pl, prm, pl.y_prev) - pl.mu_center) * pl.prior_scale; };
-    fast_mixture_points(t, sh, q.m, w.src, n, scaled, mean);
+    fast_mixture_points(t, sh, mix, w.src, scaled);
     __syncthreads();
-    fast_mixture_panels(t, q, pl.bw * pl.prior_scale);
+    fast_mixture_panels(t, q, mix, pl.bw * pl.prior_scale);
     __syncthreads();
     const int kind = PROD ? 2 : pl.transport;
     const float inv_s2 = 1.0f / (pl.sz_eff * pl.sz_eff);
     const float nu = cfg.nu;
     const float y2 = pl.y_t * pl.y_t;
-    for (int base = 0; base < n; base += nt) {
+    for (int base = s0; base < s1; base += nt) {
         const int s = base + tid;
-        const bool on = s < n;
-        const float x = w.b[min(s, n - 1)];
+        const bool on = s < s1;
+        const float x = w.xs[min(s, s1 - 1)];
         const int b = fine_bin(x) >> q.sft;
         const int j0 = t.fstart[b << q.sft];
         const bool comp = q.interpolated(b, t.fstart[(b + 1) << q.sft] - j0);
@@ -186,7 +221,7 @@ __device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_con
             den = cheb_dot(T, t.pts + kMixPts + at);
             num = cheb_dot(T, t.pts + 2 * kMixPts + at);
         } else {
-            const int r = at + (min(s, n - 1) - j0);
+            const int r = at + (min(s, s1 - 1) - j0);
             den = t.pts[kMixPts + r];
             num = t.pts[2 * kMixPts + r];
         }
@@ -195,7 +230,7 @@ __device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_con
             const int src = __ffs(todo) - 1;
             todo &= todo - 1u;
             float d_, n_;
-            mixture_warp(__shfl_sync(0xffffffffu, scaled(x), src), t, w.src, n, mean, d_, n_);
+            mixture_warp(__shfl_sync(0xffffffffu, scaled(x), src), t, w.src, d_, n_);
             if ((tid & 31) == src) {
                 den = d_;
                 num = n_;
@@ -212,50 +247,61 @@ __device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_con
         if (cfg.use_exact_gradient) glik = -0.5f + 0.5f * (nu + 1.0f) * A / opA - cfg.lik_offset;
         else glik = (logf(y2 + 1e-10f) - h + cfg.lik_offset) / 1.4f;
         const float eb = pl.fan ? 1.0f : beta;
-        w.a[s] = clampf(gp + eb * glik, -10.0f, 10.0f);
+        const float score = clampf(gp + eb * glik, -10.0f, 10.0f);
+        float curv = 0.0f;
         if (kind == 2) {
             const float hl = -0.5f * (nu + 1.0f) * A / (opA * opA);
-            w.c[s] = clampf(-(hl - inv_s2), 0.1f, 100.0f);
+            curv = clampf(-(hl - inv_s2), 0.1f, 100.0f);
+        }
+        if (alone) {
+            w.g[s] = score;
+            if (kind == 2) w.c[s] = curv;
+        } else {
+            for (int rk = 0; rk < team.size; ++rk) {
+                team.at(w.g, rk)[s] = score;
+                if (kind == 2) team.at(w.c, rk)[s] = curv;
+            }
         }
         if (last)
             io.lw[w.pidx[s]] = pl.fan ? 0.0f
                                       : pl.stc - 0.5f * h - (nu + 1.0f) * 0.5f * log1pf(fmaxf(A, -0.999f));
     }
-    __syncthreads();
+    team.sync();
     const int m = p.m, m_pad = round_up(m, 32);
-    fast_points(w.b, 1.0f, t, p, t.pts, m_pad, kHPad);
+    fast_points(w.xs, 1.0f, t, p, t.pts, m_pad, kHPad);
     for (int i = m + tid; i < m_pad; i += nt)
         t.pts[kMaxPts + i] = t.pts[2 * kMaxPts + i] = t.pts[3 * kMaxPts + i] = 0.0f;
-    auto gv = [&](int j) { return w.a[j]; };
+    auto gv = [&](int j) { return w.g[j]; };
     auto cv = [&](int j) { return w.c[j]; };
     if (kind == 2)
-        fast_weights<true, true, true>(w.b, 1.0f, t, p, t.pts + kMaxPts, t.pts + 2 * kMaxPts, t.pts + 3 * kMaxPts, gv, cv);
+        fast_weights<true, true, true>(w.xs, 1.0f, t, p, t.pts + kMaxPts, t.pts + 2 * kMaxPts, t.pts + 3 * kMaxPts, gv, cv);
     else
-        fast_weights<true, false, false>(w.b, 1.0f, t, p, t.pts + kMaxPts, t.pts + 2 * kMaxPts, nullptr, gv, cv);
+        fast_weights<true, false, false>(w.xs, 1.0f, t, p, t.pts + kMaxPts, t.pts + 2 * kMaxPts, nullptr, gv, cv);
     __syncthreads();
     if (kind == 2) {
-        if (last) fast_point_sums<true, true>(t, m, m_pad);
-        else fast_point_sums<true, false>(t, m, m_pad);
+        if (last) fast_point_sums<true, true>(t, own, m_pad);
+        else fast_point_sums<true, false>(t, own, m_pad);
     } else {
-        if (last) fast_point_sums<false, true>(t, m, m_pad);
-        else fast_point_sums<false, false>(t, m, m_pad);
+        if (last) fast_point_sums<false, true>(t, own, m_pad);
+        else fast_point_sums<false, false>(t, own, m_pad);
     }
     __syncthreads();
     if (kind == 2) {
-        fast_coefficients(t, p.nc, 4, last ? 7 : 5);
+        fast_coefficients(t, own.c0, own.c1, 4, last ? 7 : 5);
     } else {
-        fast_coefficients(t, p.nc, 4, 2);
-        if (last) fast_coefficients(t, p.nc, 9, 2);
+        fast_coefficients(t, own.c0, own.c1, 4, 2);
+        if (last) fast_coefficients(t, own.c0, own.c1, 9, 2);
     }
     __syncthreads();
     const float sign = cfg.stein_repulsive_sign == 1 ? 1.0f : -1.0f;
     const float inv_bw = pl.inv_bw, inv_bw2 = pl.inv_bw2, inv_n = 1.0f / (float)n;
     const float es = pl.eps_step * bf, rr = cfg.rmsprop_rho;
     ksd = 0.0f;
-    for (int s = tid; s < n; s += nt) {
-        const float x = w.b[s];
+    for (int s = s0 + tid; s < s1; s += nt) {
+        const float x = w.xs[s];
         const int i = w.pidx[s];
-        const float v0 = io.v[i];
+        // a particle's member may change between iterations: its moment lives in L2
+        const float v0 = alone ? io.v[i] : __ldcg(io.v + i);
         const int b = fine_bin(x) / kFine;
         const int j0 = t.fstart[kFine * b];
         float sum[7] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
@@ -282,24 +328,30 @@ __device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_con
         }
         float phi = (sum[0] + sign * 2.0f * inv_bw * sum[1]) * inv_n;
         if (kind == 2) {
-            const float nk = sum[4] + 2.0f * fast_window(x, w.b, t, p);
+            const float nk = sum[4] + 2.0f * fast_window(x, w.xs, t, p);
             float H = (sum[3] + 2.0f * inv_bw2 * nk) / fmaxf(sum[2], 1e-6f);
             H = clampf(H, 0.1f, 100.0f);
             phi = phi * (1.0f / H) * 0.7f;
         }
         if (last) {
-            const float si = w.a[s];
+            const float si = w.g[s];
             ksd += si * sum[0] + 2.0f * inv_bw * (si * sum[1] - sum[5]) + 2.0f * inv_bw2 * sum[6];
         }
         const float vn = rr * v0 + (1.0f - rr) * phi * phi;
-        io.v[i] = vn;
+        if (alone) io.v[i] = vn;
+        else __stcg(io.v + i, vn);
         const float drift = es * phi * rsqrtf(vn + cfg.rmsprop_eps);
         float diff = 0.0f;
         if (pl.temp > 1e-6f) diff = sqrtf(2.0f * es * pl.temp) * nz.normal(i, kn);
         const float h_new = clamp_h(fmaf(x, pl.bw, pl.center) + drift + diff);
-        w.c[i] = (h_new - pl.center) * inv_bw;
+        const float hs_new = (h_new - pl.center) * inv_bw;
+        if (alone) {
+            w.xn[i] = hs_new;
+        } else {
+            for (int rk = 0; rk < team.size; ++rk) team.at(w.xn, rk)[i] = hs_new;
+        }
     }
-    __syncthreads();
+    team.sync();
     return true;
 }
 
@@ -311,7 +363,7 @@ __device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_con
 // caller guarantees full-Newton transport, Gaussian state noise and no Heun
 // step (the production configuration), so only those code paths are compiled
 // and the kernel body stays small (instruction fetch bounds the latency kernel).
-// FAST: the Stein iterations go through the fast sums (one CTA, Gaussian state
+// FAST: the Stein iterations go through the fast sums (Gaussian state
 // noise, vanilla or full-Newton transport, no Heun step, dynamic shared memory
 // of fast_smem_floats); a tick whose particles do not fit them finishes with
 // the <R, S> sweeps.  NT: threads of the CTA (no Heun step above kThreads).
@@ -323,11 +375,7 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
     const int n = sm.n;
     FastWork fw;
     if constexpr (FAST) {
-        fw.a = sm.h[0];
-        fw.b = sm.h[1];
-        fw.c = sm.g;
-        fw.pidx = reinterpret_cast<unsigned short*>(sm.c);
-        fw.tab = carve_fast(sm.c + sm.np / 2, sm.np, true);
+        carve_fast_work(fw, sm, team.size > 1);
         fast_load_tables(fw.tab);
     }
     if (tid == 0) {
@@ -481,16 +529,23 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
     bool direct = !FAST;
     if constexpr (FAST) {
         if (budget > 0) {
-            bool fits = fast_sources(fw, pl, n, *fsh);
+            bool fits = fast_sources(fw, pl, io, *fsh);
+            if (team.size > 1) team.sync();   // no member reads its means any more
             while (fits && it0 < budget) {
                 const float beta = pl.beta[stage_of(pl, it0)];
                 float kt;
-                fits = fast_iteration<PROD>(fw, pl, cfg, prm, io, nz, kn, beta, sqrtf(beta), it0 == budget - 1, *fsh, kt);
+                fits = fast_iteration<PROD>(fw, pl, cfg, io, nz, kn, beta, sqrtf(beta), it0 == budget - 1,
+                                            team, *fsh, kt);
                 if (!fits) break;
-                if (it0 == budget - 1) ksd_publish<NT>(kt, pl, team);
-                float* x = fw.c;
-                fw.c = fw.a;
-                fw.a = x;
+                if (it0 == budget - 1) {
+                    ksd_publish<NT>(kt, pl, team);
+                    if (team.size > 1) team.sync();
+                }
+                if (team.size == 1) {
+                    float* x = fw.xn;
+                    fw.xn = fw.c = fw.x;
+                    fw.x = fw.g = x;
+                }
                 if (pl.temp > 1e-6f) ++kn;
                 ++it0;
             }
@@ -498,16 +553,17 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
                 // the sweeps take over: positions, prior means (sorted) and moments where they expect them
                 __syncthreads();
                 direct = true;
-                if (fw.a != sm.h[0])
-                    for (int i = tid; i < n; i += NT) sm.h[0][i] = fw.a[i];
+                if (fw.x != sm.h[0])
+                    for (int i = tid; i < n; i += NT) sm.h[0][i] = fw.x[i];
                 __syncthreads();
                 pads();
                 for (int i = tid; i < n; i += NT) {
                     sm.mu[i] = (prior_mean(io.h[i], pl, prm, y_prev) - pl.mu_center) * pl.prior_scale;
-                    sm.v[i] = io.v[i];
                 }
+                for (int li = tid; li < sm.row1 - sm.row0; li += NT) sm.v[li] = __ldcg(io.v + sm.row0 + li);
                 __syncthreads();
                 bitonic_sort(sm.mu, sm.p2);
+                if (team.size > 1) team.sync();
             }
         }
     }
@@ -599,7 +655,7 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
     // ---- back to log-volatility coordinates
     float* hf = sm.h[cur];
     if constexpr (FAST)
-        if (!direct) hf = fw.a;
+        if (!direct) hf = fw.x;
     if (budget > 0) {
         for (int i = tid; i < n; i += NT) hf[i] = fmaf(hf[i], pl.bw, pl.center);
         __syncthreads();

@@ -179,9 +179,9 @@ __device__ inline void fast_transport_2f(const Smem& f, float* __restrict__ v, c
     fast_weights<true, false, false>(w.xs, 1.0f, t, p, t.pts + kMaxPts2f, t.pts + 2 * kMaxPts2f, nullptr,
                                      [&](int j) { return g[w.pidx[j]]; }, [](int) { return 0.0f; });
     __syncthreads();
-    fast_point_sums<false, false, kMaxPts2f, 3>(t, p.m, m_pad);
+    fast_point_sums<false, false, kMaxPts2f, 3>(t, all_points(p), m_pad);
     __syncthreads();
-    fast_coefficients<kMaxPts2f>(t, p.nc, 3, 2);
+    fast_coefficients<kMaxPts2f>(t, 0, p.nc, 3, 2);
     __syncthreads();
     // the next particle's moment is fetched while one is moved
     int i_next = w.pidx[min(tid, n - 1)];

@@ -96,6 +96,61 @@ def test_fast_sums_match_oracle(pkg, oracle_mod, newton, sigma):
     b.close()
 
 
+@pytest.mark.parametrize("newton", [1, 0])
+@pytest.mark.parametrize("kind", STATES)
+def test_single_filter_fast_sums_match_oracle(pkg, oracle_mod, newton, kind):
+    """The same for a single filter, whose cluster shares the sums: sizes
+    around the first that takes them, ones that leave a member fewer slots
+    than the others, and a spread that makes all members turn to the sweeps."""
+    ns = [2047, 2048, 2049, 3001, 4096] + ([8192] if kind in ("cloud", "spread") else [])
+    cfg = pkg.production_config(8.0, 5)
+    cfg.update(use_newton=newton, use_full_newton=newton, stein_min_steps=4, stein_max_steps=5)
+    for n in ns:
+        rng = np.random.default_rng(n)
+        f = pkg.SVPF(n, 5, 8.0)
+        f.configure(**cfg.to_dict())
+        f.initialize(0.95, 0.05, -1.0, -0.2, seed=3)
+        ctl = f.get_state()[0]
+        ctl.timestep, ctl.ksd_prev, ctl.ksd_last, ctl.vol_prev = 12, 0.6, 0.6, 0.6
+        ctl.guide_initialized, ctl.h_mean_prev, ctl.bw_sq = 1, -1.0, 0.04
+        ctl.return_ema, ctl.return_var = 0.5, 0.3
+        h = _state(kind, n, rng, -1.0)
+        v = rng.uniform(0.05, 0.5, n).astype(np.float32)
+        f.set_state(ctl, h, (h - 0.1).astype(np.float32), v, np.zeros(n, np.float32))
+        nrm, uni = tape.tape(5, 0, n, 16, 2)
+        f.set_noise_tape(nrm, uni)
+        twin = _twin(oracle_mod, _One(f), 0, cfg, (0.95, 0.05, -1.0, -0.2))
+        mirrors = []
+        for nudge in (0.0, 2.0 ** -22, -(2.0 ** -22)):
+            o = _twin(oracle_mod, _One(f), 0, cfg, (0.95, 0.05, -1.0, -0.2), 1)
+            o.h = o.h * (1.0 + nudge)
+            mirrors.append(o)
+        y = 25.0 if kind == "shock" else 0.4
+        rc, out = f.step_raw(y, 0.3)
+        with cf.ThreadPoolExecutor(max_workers=4) as pool:
+            want, *around = pool.map(lambda o: o.step(y, 0.3, nrm, uni), [twin] + mirrors)
+        ctl, got = f.get_state()[:2]
+        assert rc == 0 and ctl.status == 0 and ctl.stein_steps_used == want.steps_used, n
+        dev = max(rel_err(m.h, twin.h) for m in mirrors)
+        assert rel_err(got, twin.h) < max(TOL, 4 * dev), (n, rel_err(got, twin.h), dev)
+        for name, value, base in (("loglik", out.loglik, TOL), ("vol", out.vol, TOL), ("h_mean", out.h_mean, TOL),
+                                  ("ksd", ctl.ksd_last, 1e-3)):
+            w = getattr(want, name)
+            dev = max(abs(getattr(a, name) - w) for a in around) / max(1.0, abs(w))
+            assert abs(value - w) < max(base, 4 * dev) * max(1.0, abs(w)), (n, name, value, w, dev)
+        f.close()
+
+
+class _One:
+    """A single filter's state in the form that a batch gives it."""
+
+    def __init__(self, f):
+        self.f = f
+
+    def get_state(self, _):
+        return self.f.get_state()
+
+
 @pytest.mark.parametrize("exact", [1, 0])
 def test_two_factor_fast_sums_match_oracle(pkg, oracle_mod, exact):
     """The same for the two-factor tick's transports: both factors of made
