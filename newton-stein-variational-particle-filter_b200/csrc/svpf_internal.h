@@ -191,7 +191,7 @@ SVPF_HD inline bool config_loops_ok(const svpf_config_t& c) {
 // the batch kernel for n particles.
 int default_single_tile(int n, int C);
 int default_batch_tile(int n);
-// Default cluster size of the single-filter kernel for n particles.
+// Default cluster size of the single-filter kernels for n particles.
 int default_cluster(int n);
 
 cudaError_t launch_single(const SingleArgs& a, int C, int tile, cudaStream_t s);

@@ -135,9 +135,17 @@ cudaError_t configure_kernel(const void* func, int dyn_smem_bytes, bool nonporta
     return cudaSuccess;
 }
 
+// One CTA up to 64 rows (a cluster's barriers and pushes cost more than the
+// rows), above that the smallest cluster of four or more whose members take
+// their rows in one sweep of the eight-lane tile (32 rows).  Measured on B200,
+// us per call on 1 / 2 / 4 / 8 / 16 CTAs, production settings: N = 64 41/46/46/47/-,
+// 100 47/48/45/46/-, 200 -/-/47/44/48, 256 -/-/48/45/45, 300 -/-/61/53/51,
+// 500 -/-/74/61/54; two factors: 64 116/127/124/127/-, 200 -/-/171/152/157,
+// 300 -/-/276/209/184, 511 -/-/376/259/209.
 int default_cluster(int n) {
-    int C = 1;
-    while (C < kMaxCluster && n / (2 * C) >= 32) C <<= 1;
+    constexpr int kRows = kThreads / 8;
+    int C = n <= 2 * kRows ? 1 : 4;
+    while (C > 1 && C < kMaxCluster && n > kRows * C) C <<= 1;
     return C;
 }
 

@@ -569,7 +569,8 @@ size_t v2_smem_cap() {
 }
 
 int v2_cluster(int n) {
-    int C = default_cluster(n);
+    int C = 1;
+    while (C < 16 && n / (2 * C) >= 32) C <<= 1;
     while (C > 1 && v2_smem_bytes(n, C, 0) > v2_smem_cap()) C >>= 1;
     return C;
 }
