@@ -884,7 +884,8 @@ def main():
     # 2 MUFU evaluations (ex2, rcp) and 13 FP32 operations.  Nominal rates
     # 16 MUFU and 128 FP32 results per clock per SM -> 8 pair-iterations per
     # clock per SM (MUFU-bound); the peak used is the same bound from the
-    # rates measured on this GPU (svpf_measure_pipe_rates), the nominal beside it
+    # rates measured on this GPU (svpf_measure_pipe_rates), the nominal beside it.
+    # It bounds a summation over all pairs; the fast sums (csrc/svpf_fast.cuh) go past it.
     PAIRS_PER_CLK_NOMINAL = min(16.0 / 2.0, 128.0 / 13.0)
     try:
         rates = pkg.pipe_rates()
@@ -936,14 +937,17 @@ def main():
                     "timing": "host wall clock around each svpf_batch_step call (host y in, host outputs back), "
                               "same ticks as the device-timed steps"},
             "gpu_launches": launches,
-            "roofline": {"bound": "fp32+mufu", "achieved": achieved, "peak": peak, "unit": "Gpair/s",
+            "roofline": {"bound": "fp32+mufu of the direct pair sums", "achieved": achieved, "peak": peak, "unit": "Gpair/s",
                          "frac": achieved / peak, "traffic": traffic, "peak_source": peak_src,
                          "pipe_rates": rates, "peak_nominal": peak_nominal,
                          "note": "pair = one (i,j) Stein iteration: mixture-prior pair + transport pair (2 MUFU "
                                  "evaluations, 13 FP32 ops); peak = "
                                  f"{sms} SMs x {sm_mhz:.0f} MHz (sampled) x min(MUFU/2, FP32/13) pair/clk/SM from "
                                  "the MUFU and FP32 results per SM clock measured on this GPU "
-                                 "(nominal 16 and 128: 8 pair/clk/SM)"},
+                                 "(nominal 16 and 128: 8 pair/clk/SM).  The tick does not evaluate every pair: filters "
+                                 "of 257 particles or more take the same sums from interpolated panels (far fewer "
+                                 "kernel evaluations, FP32 accuracy), so achieved counts the pairs that the sums stand "
+                                 "for and frac says how far the tick is beyond what a direct summation could reach"},
             "pair_iterations_per_s": achieved * 1e9,
             "single_filter_latency": lat,
             "plain_step_loop": plain,

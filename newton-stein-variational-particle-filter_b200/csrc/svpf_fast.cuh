@@ -42,11 +42,12 @@
 // 250 k cycles (the window 88 k of them: about 36 kernel values per particle;
 // point sums 31 k, rows 27 k, mixture points 22 k, binning 16 k, weights 12 k)
 // against 4.7 M with the sweeps, one of N = 512 55 k against 100 k.  The batch
-// tick of 4096 filters (N 256 to 4096) went from 83.6 to 4.7 ms, its first
-// tick from 83 to 13 ms, 300 filters of 100 to 1500 particles from 4.0 to
-// 0.52 ms.  The two-factor tick's transports (no mixture, no Hessian) take the
+// tick of 4096 filters (N 256 to 4096) went from 83.7 to 4.8 ms, its first
+// tick from 83 to 12 ms, 300 filters of 100 to 1500 particles from 4.0 to
+// 0.37 ms (CTAs of 512 threads), one filter of 4096 on a cluster from 0.68 to
+// 0.22 ms.  The two-factor tick's transports (no mixture, no Hessian) take the
 // same way: a request round of 200 instruments of 256 to 2048 particles went
-// from 7.5 to 2.9 ms, bound by the ticks of N = 2048.
+// from 7.5 to 1.9 ms, bound by the ticks of N = 2048.
 #pragma once
 
 #include "svpf_device.cuh"
