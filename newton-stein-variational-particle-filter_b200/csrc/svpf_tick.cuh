@@ -456,6 +456,21 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
             st[3] = fmaxf(st[3], hp);
         }
     }
+    if constexpr (NT != kThreads) {
+        // The moments in the order of a CTA of kThreads, so that the centre and
+        // the bandwidth do not depend on the CTA's width: a particle at the
+        // position clamp keeps the same last bit, which the next tick's
+        // comparison of h with h_prev (asymmetric rho) can turn on.
+        __syncthreads();
+        st[0] = st[1] = 0.0f;
+        if (tid < kThreads) {
+            for (int i = tid; i < n; i += kThreads) {
+                const float hp = sm.h[0][i];
+                st[0] += hp;
+                st[1] += hp * hp;
+            }
+        }
+    }
     if constexpr (FAST) {
         const int op[5] = {0, 0, 2, 1, 0};
         block_reduce<5, NT>(st, op, pl);
