@@ -165,7 +165,7 @@ struct Plan {
     FactorPlan fac[2];     // two-factor: fast, slow
     float fmean[2];        // two-factor: factor means of the previous tick (guide)
     float gmean2[2];       // two-factor: EKF guide means
-    float red[5][16];      // block reduction scratch, a value per warp
+    float red[4][kWarps];  // block reduction scratch
     float ksd_slot[kMaxCluster];
 };
 
@@ -319,21 +319,31 @@ __device__ __forceinline__ float warp_min(float v) {
     return v;
 }
 
-// Reduce up to five values (op per slot: 0 sum, 1 max, 2 min); result visible
-// to all threads.  Contains two __syncthreads.
+// First item of a thread in a sum over items in strides of kThreads: the
+// threads above kThreads have none (end: the number of items).
+template <int NT>
+__device__ __forceinline__ int first_lane(int end) {
+    return NT == kThreads || threadIdx.x < kThreads ? (int)threadIdx.x : end;
+}
+
+// Reduce up to four values (op per slot: 0 sum, 1 max, 2 min); result visible
+// to all threads.  Contains two __syncthreads.  A CTA of more than kThreads
+// threads sums in the order of one of kThreads: its first kThreads threads hold
+// the values (first_lane), the others only take the result.  With it a filter's
+// bits do not depend on the CTA it ran on, and so on the launch's other filters.
 template <int K, int NT = kThreads>
 __device__ __forceinline__ void block_reduce(float (&v)[K], const int (&op)[K], Plan& pl) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         v[k] = op[k] == 0 ? warp_sum(v[k]) : op[k] == 1 ? warp_max(v[k]) : warp_min(v[k]);
-        if (lane == 0) pl.red[k][w] = v[k];
+        if (lane == 0 && (NT == kThreads || w < kWarps)) pl.red[k][w] = v[k];
     }
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         float a = pl.red[k][0];
-        for (int i = 1; i < NT / 32; ++i) {
+        for (int i = 1; i < kWarps; ++i) {
             const float b = pl.red[k][i];
             a = op[k] == 0 ? a + b : op[k] == 1 ? fmaxf(a, b) : fminf(a, b);
         }

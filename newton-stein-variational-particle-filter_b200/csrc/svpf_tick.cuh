@@ -174,12 +174,14 @@ __device__ inline bool fast_sources(FastWork& w, const Plan& pl, const FilterIO&
 // One Stein iteration of a filter through the fast sums (svpf_fast.cuh): gradient pass (svpf_opt_kernels.cu:354-521), vanilla or
 // full-Newton transport (:527-1103) as grad_pass and transport_pass take it.
 // Positions: w.x before, w.xn after (w.x untouched when it returns false: the
-// particles do not fit the tables).  ksd: this thread's KSD terms.
+// particles do not fit the tables).  ksd: this thread's KSD terms (each slot's
+// term takes its score's place, which only that slot's thread still reads, and
+// is summed from there in the order of block_reduce).
 // In a cluster every member bins all particles (a copy of the same work: it
 // costs less than exchanging the order) and sums at the points and moves the
 // particles of its own slots; scores, curvatures and new positions go to every
 // member through distributed shared memory, one cluster barrier after each.
-template <bool PROD>
+template <bool PROD, int NT>
 __device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_config_t& cfg,
                                const FilterIO& io, const Noise& nz, int kn, float beta, float bf, bool last,
                                const Team& team, FastSh& sh, float& ksd) {
@@ -335,7 +337,7 @@ __device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_con
         }
         if (last) {
             const float si = w.g[s];
-            ksd += si * sum[0] + 2.0f * inv_bw * (si * sum[1] - sum[5]) + 2.0f * inv_bw2 * sum[6];
+            w.g[s] = si * sum[0] + 2.0f * inv_bw * (si * sum[1] - sum[5]) + 2.0f * inv_bw2 * sum[6];
         }
         const float vn = rr * v0 + (1.0f - rr) * phi * phi;
         if (alone) io.v[i] = vn;
@@ -352,6 +354,8 @@ __device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_con
         }
     }
     team.sync();
+    if (last)
+        for (int s = s0 + first_lane<NT>(s1); s < s1; s += kThreads) ksd += w.g[s];
     return true;
 }
 
@@ -395,7 +399,14 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
 
     // ---- predict (svpf_opt_kernels.cu:125-276), guide (:282-327), prior means
     //      (:384-392); every team member does all N rows, no exchange needed.
-    float st[FAST ? 5 : 4] = {0.0f, 0.0f, 1e10f, -1e10f};
+    float st[4] = {0.0f, 0.0f, 1e10f, -1e10f};
+    float sum_mk[1] = {0.0f};
+    auto moments = [&](float hp) {
+        st[0] += hp;
+        st[1] += hp * hp;
+        st[2] = fminf(st[2], hp);
+        st[3] = fmaxf(st[3], hp);
+    };
     {
         const float hbar = ctl.h_mean_prev;
         const bool mim = cfg.use_mim || cfg.use_guided;
@@ -446,37 +457,26 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
             if constexpr (FAST) {
                 const float mk = prior_mean(hi, pl, prm, y_prev);
                 sm.g[i] = mk;
-                st[4] += mk;
+                if constexpr (NT == kThreads) sum_mk[0] += mk;
             } else {
                 sm.mu[i] = pl.mu_eff + prm.rho * (hi - pl.mu_eff) + prm.gamma * y_prev / (expf(hi * 0.5f) + 1e-8f);
             }
-            st[0] += hp;
-            st[1] += hp * hp;
-            st[2] = fminf(st[2], hp);
-            st[3] = fmaxf(st[3], hp);
+            if constexpr (NT == kThreads) moments(hp);
         }
     }
     if constexpr (NT != kThreads) {
-        // The moments in the order of a CTA of kThreads, so that the centre and
-        // the bandwidth do not depend on the CTA's width: a particle at the
-        // position clamp keeps the same last bit, which the next tick's
-        // comparison of h with h_prev (asymmetric rho) can turn on.
+        // in the order of a CTA of kThreads (block_reduce)
         __syncthreads();
-        st[0] = st[1] = 0.0f;
-        if (tid < kThreads) {
-            for (int i = tid; i < n; i += kThreads) {
-                const float hp = sm.h[0][i];
-                st[0] += hp;
-                st[1] += hp * hp;
-            }
+        for (int i = first_lane<NT>(n); i < n; i += kThreads) {
+            moments(sm.h[0][i]);
+            if constexpr (FAST) sum_mk[0] += sm.g[i];
         }
     }
-    if constexpr (FAST) {
-        const int op[5] = {0, 0, 2, 1, 0};
-        block_reduce<5, NT>(st, op, pl);
-    } else {
+    {
         const int op[4] = {0, 0, 2, 1};
         block_reduce<4, NT>(st, op, pl);
+        const int add[1] = {0};
+        if constexpr (FAST) block_reduce<1, NT>(sum_mk, add, pl);
     }
     // ---- bandwidth (svpf_fused_bandwidth_kernel, svpf_opt_kernels.cu:1159-1235)
     if (tid == 0) {
@@ -503,7 +503,7 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
         pl.inv_bw = 1.0f / bw;
         pl.inv_bw2 = 1.0f / (bw * bw);
         pl.center = mean;
-        if constexpr (FAST) pl.mu_center = st[4] * inv_n;   // the panels of the prior means are centred on them
+        if constexpr (FAST) pl.mu_center = sum_mk[0] * inv_n;   // the panels of the prior means are centred on them
         else pl.mu_center = pl.mu_eff;
         pl.prior_scale = sqrtf(kLog2e * 0.5f / (pl.sz_eff * pl.sz_eff));
     }
@@ -549,7 +549,7 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
             while (fits && it0 < budget) {
                 const float beta = pl.beta[stage_of(pl, it0)];
                 float kt;
-                fits = fast_iteration<PROD>(fw, pl, cfg, io, nz, kn, beta, sqrtf(beta), it0 == budget - 1,
+                fits = fast_iteration<PROD, NT>(fw, pl, cfg, io, nz, kn, beta, sqrtf(beta), it0 == budget - 1,
                                             team, *fsh, kt);
                 if (!fits) break;
                 if (it0 == budget - 1) {
@@ -691,13 +691,13 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
 
     // ---- outputs (svpf_fused_outputs_kernel, svpf_opt_kernels.cu:1109-1153)
     float mx[1] = {-1e10f};
-    for (int i = tid; i < n; i += NT) mx[0] = fmaxf(mx[0], io.lw[i]);
+    for (int i = first_lane<NT>(n); i < n; i += kThreads) mx[0] = fmaxf(mx[0], io.lw[i]);
     {
         const int op[1] = {1};
         block_reduce<1, NT>(mx, op, pl);
     }
     float acc[3] = {0.0f, 0.0f, 0.0f};
-    for (int i = tid; i < n; i += NT) {
+    for (int i = first_lane<NT>(n); i < n; i += kThreads) {
         acc[0] += ex2_approx((io.lw[i] - mx[0]) * kLog2e);
         acc[1] += expf(fminf(hf[i] * 0.5f, 20.0f));
         acc[2] += hf[i];

@@ -239,6 +239,12 @@ __device__ void run_tick_2f(const svpf_config_t& cfg, const SVPFParams& prm, svp
     //      guide (svpf_apply_guide_two_factor_kernel, :321-362); every member
     //      does all rows.
     float st[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    auto moments = [&](float hf, float hs) {
+        st[0] += hf;
+        st[1] += hf * hf;
+        st[2] += hs;
+        st[3] += hs * hs;
+    };
     {
         const float rf = cfg.rho_fast, sf = cfg.sigma_fast, rs = cfg.rho_slow, ss = cfg.sigma_slow;
         const float gs = pl.gs;
@@ -268,11 +274,13 @@ __device__ void run_tick_2f(const svpf_config_t& cfg, const SVPFParams& prm, svp
             }
             sm.f[0].h[0][i] = hf;
             sm.f[1].h[0][i] = hs;
-            st[0] += hf;
-            st[1] += hf * hf;
-            st[2] += hs;
-            st[3] += hs * hs;
+            if constexpr (NT == kThreads) moments(hf, hs);
         }
+    }
+    if constexpr (NT != kThreads) {
+        // in the order of a CTA of kThreads (block_reduce)
+        __syncthreads();
+        for (int i = first_lane<NT>(n); i < n; i += kThreads) moments(sm.f[0].h[0][i], sm.f[1].h[0][i]);
     }
     {
         const int op[4] = {0, 0, 0, 0};
@@ -341,13 +349,13 @@ __device__ void run_tick_2f(const svpf_config_t& cfg, const SVPFParams& prm, svp
     const float* hf = sm.f[0].h[cur];
     const float* hs = sm.f[1].h[cur];
     float mx[1] = {-1e30f};
-    for (int i = tid; i < n; i += NT) mx[0] = fmaxf(mx[0], io.lw[i]);
+    for (int i = first_lane<NT>(n); i < n; i += kThreads) mx[0] = fmaxf(mx[0], io.lw[i]);
     {
         const int op[1] = {1};
         block_reduce<1, NT>(mx, op, pl);
     }
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    for (int i = tid; i < n; i += NT) {
+    for (int i = first_lane<NT>(n); i < n; i += kThreads) {
         acc[0] += expf(io.lw[i] - mx[0]);
         acc[1] += hf[i];
         acc[2] += hs[i];
