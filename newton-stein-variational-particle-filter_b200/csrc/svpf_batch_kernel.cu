@@ -30,7 +30,6 @@ __global__ void __launch_bounds__(NT, 2 * kThreads / NT) batch_tick_kernel(const
     __shared__ svpf_config_t cfg;
     __shared__ SVPFParams prm;
     __shared__ svpf_out_t out;
-    __shared__ FastSh fsh;
     __shared__ int s_next;
     const Team team{0, 1};
     for (;;) {
@@ -61,7 +60,7 @@ __global__ void __launch_bounds__(NT, 2 * kThreads / NT) batch_tick_kernel(const
             const float ypr = readable_y_prev(yp);
             const int tile = a.tile[f];
             if (tile & kTileFast) {
-                run_tick<2, 1, false, PROD, 0, true, NT>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out, &fsh);
+                run_tick<2, 1, false, PROD, 0, true, NT>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out);
             } else if constexpr (NT == kThreads) {
                 switch (tile) {
                     case 1: run_tick<1, 4, false, PROD>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;
@@ -96,7 +95,6 @@ __global__ void __launch_bounds__(NT, 2 * kThreads / NT) batch_tick_2f_kernel(co
     __shared__ svpf_config_t cfg;
     __shared__ SVPFParams prm;
     __shared__ svpf_out_t out;
-    __shared__ FastSh fsh;
     __shared__ int s_next;
     const Team team{0, 1};
     for (;;) {
@@ -123,7 +121,7 @@ __global__ void __launch_bounds__(NT, 2 * kThreads / NT) batch_tick_2f_kernel(co
         if (!refuse_nonfinite(yt, ctl, out)) {   // a refused tick leaves the filter as it was
             const float ypr = readable_y_prev(yp);
             if (tile & kTileFast) {
-                run_tick_2f<1, 1, true, NT>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out, &fw, &fsh);
+                run_tick_2f<1, 1, true, NT>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out, &fw);
             } else if constexpr (NT == kThreads) {
                 switch (tile) {
                     case 1: run_tick_2f<1, 4>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;

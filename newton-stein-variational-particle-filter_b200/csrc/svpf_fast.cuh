@@ -137,6 +137,14 @@ struct Panels {
     __device__ __forceinline__ float local(float x, int b) const { return (x - centre(b)) * (kInvHalfW * narrow); }
 };
 
+// Shared scalars, behind the tables: a static variable would take them from
+// every kernel's dynamic shared memory limit (max_dyn_smem).
+struct FastSh {
+    unsigned scan[kMaxWarps];
+    int over;                 // points do not fit
+    int n_far;                // mixture points far from every mean, listed in pref's space
+};
+
 // Shared-memory tables of the fast sums (dynamic part: fast_table_floats()).
 struct FastTab {
     float* basis;             // kBasis, then kNode
@@ -153,19 +161,15 @@ struct FastTab {
     unsigned short* mpt;      // mixture panels: first points, [kFineBins]
     unsigned short* mcomp;    // [kMixComp]
     unsigned char* bad;       // [kMixComp] mixture panel not interpolated
+    FastSh* sh;
 };
-// Static shared scalars.
-struct FastSh {
-    unsigned scan[kMaxWarps];
-    int over;                 // points do not fit
-    int n_far;                // mixture points far from every mean, listed in pref's space
-};
-
 constexpr int kTabBasis = kP * kP + 16;
 constexpr int kTabPts = kPtRows * kMaxPts;
 constexpr int kTabPref = kMaxComp * kFine * kP;
+// (an even number: FastSh follows)
 constexpr int kTabShorts = (kFineBins + 8) + 2 * (kFineBins / kFine + 8) + 2 * (kFineBins / kFine) + kFineBins +
                            2 * kMixComp;
+static_assert(kTabShorts % 2 == 0 && sizeof(FastSh) % sizeof(float) == 0, "FastSh behind the tables");
 // binning counters and ranks take the points' space and the one behind it
 static_assert(kMixPts / 2 <= kTabPref, "the list of far points takes pref's space");
 static_assert(kBinWarps * kFineBins / 2 + SVPF_MAX_PARTICLES / 2 <= kTabPts + kTabPref && 4 * kMixPts <= kTabPts,
@@ -178,7 +182,7 @@ __host__ __device__ inline int fast_points_floats(int np, bool mixture) {
 }
 __host__ __device__ inline int fast_table_floats(int np, bool mixture) {
     return round_up(kTabBasis + fast_points_floats(np, mixture) + kTabShorts / 2 + 8 +
-                        (mixture ? kTabPref + 2 * kMaxSrc : 0), 16);
+                        (int)(sizeof(FastSh) / sizeof(float)) + (mixture ? kTabPref + 2 * kMaxSrc : 0), 16);
 }
 
 __device__ inline FastTab carve_fast(float* p, int np, bool mixture) {
@@ -212,6 +216,7 @@ __device__ inline FastTab carve_fast(float* p, int np, bool mixture) {
     t.mcomp = q;
     q += kMixComp;
     t.bad = reinterpret_cast<unsigned char*>(q);
+    t.sh = reinterpret_cast<FastSh*>(p + kTabShorts / 2);
     return t;
 }
 

@@ -106,7 +106,7 @@ size_t max_dyn_smem() {
         int v = 0;
         if (cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
         const size_t static_bytes = sizeof(Plan) + sizeof(svpf_ctl_t) + sizeof(svpf_config_t) +
-                                    sizeof(SVPFParams) + sizeof(svpf_out_t) + sizeof(FastSh) + 64;
+                                    sizeof(SVPFParams) + sizeof(svpf_out_t) + 64;
         g_max_dyn_smem[dev] = (size_t)v > static_bytes ? (size_t)v - static_bytes : 0;
     }
     return g_max_dyn_smem[dev];

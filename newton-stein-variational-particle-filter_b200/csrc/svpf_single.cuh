@@ -78,7 +78,6 @@ __global__ void __launch_bounds__(kWideThreads, 1) single_fast_kernel(const __gr
     __shared__ svpf_config_t cfg;
     __shared__ SVPFParams prm;
     __shared__ svpf_out_t out;
-    __shared__ FastSh fsh;
     cg::cluster_group cl = cg::this_cluster();
     const Team team{(int)cl.block_rank(), (int)cl.num_blocks()};
     copy_words<kWideThreads>(&ctl, &a.ctl);
@@ -96,7 +95,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) single_fast_kernel(const __gr
     }
     if (!refuse_nonfinite(a.y_t, ctl, out)) {   // every member sees the same y_t
         run_tick<1, 1, false, PROD, 0, true, kWideThreads>(cfg, prm, ctl, a.y_t, readable_y_prev(a.y_prev), io, nz, sm,
-                                                           pl, team, out, &fsh);
+                                                           pl, team, out);
         flag_y_prev(a.y_prev, ctl);
     }
     if (team.rank == 0) {

@@ -374,7 +374,7 @@ __device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_con
 template <int R, int S, bool SCAN = false, bool PROD = false, int U = 0, bool FAST = false, int NT = kThreads>
 __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_ctl_t& ctl, float y_t,
                          float y_prev, const FilterIO& io, const Noise& nz, const Smem& sm, Plan& pl,
-                         const Team& team, svpf_out_t& out, FastSh* fsh = nullptr) {
+                         const Team& team, svpf_out_t& out) {
     const int tid = threadIdx.x;
     const int n = sm.n;
     FastWork fw;
@@ -544,13 +544,13 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
     bool direct = !FAST;
     if constexpr (FAST) {
         if (budget > 0) {
-            bool fits = fast_sources(fw, pl, io, *fsh);
+            bool fits = fast_sources(fw, pl, io, *fw.tab.sh);
             if (team.size > 1) team.sync();   // no member reads its means any more
             while (fits && it0 < budget) {
                 const float beta = pl.beta[stage_of(pl, it0)];
                 float kt;
                 fits = fast_iteration<PROD, NT>(fw, pl, cfg, io, nz, kn, beta, sqrtf(beta), it0 == budget - 1,
-                                            team, *fsh, kt);
+                                            team, *fw.tab.sh, kt);
                 if (!fits) break;
                 if (it0 == budget - 1) {
                     ksd_publish<NT>(kt, pl, team);

@@ -135,9 +135,10 @@ __device__ inline Smem2 carve_2f_fast(float* base, int n, FastWork2& w) {
 // log-volatility units; the sums run in bandwidths from the factor's mean.  A
 // step whose particles do not fit the tables sweeps over the pairs.
 __device__ inline void fast_transport_2f(const Smem& f, float* __restrict__ v, const FastWork2& w, const FactorPlan& fp,
-                                         const svpf_config_t& cfg, float beta, const Noise& nz, int kn, FastSh& sh) {
+                                         const svpf_config_t& cfg, float beta, const Noise& nz, int kn) {
     const int tid = threadIdx.x, nt = blockDim.x, n = f.n;
     const FastTab& t = w.tab;
+    FastSh& sh = *t.sh;
     float* x = f.h[0];
     const float* g = f.g;
     const float ib = fp.inv_bw, cen = fp.center;
@@ -216,7 +217,7 @@ __device__ inline void fast_transport_2f(const Smem& f, float* __restrict__ v, c
 template <int R, int S, bool FAST = false, int NT = kThreads>
 __device__ void run_tick_2f(const svpf_config_t& cfg, const SVPFParams& prm, svpf_ctl_t& ctl, float y_t,
                             float y_prev, const FilterIO& io, const Noise& nz, const Smem2& sm, Plan& pl,
-                            const Team& team, svpf_out_t& out, const FastWork2* fw = nullptr, FastSh* fsh = nullptr) {
+                            const Team& team, svpf_out_t& out, const FastWork2* fw = nullptr) {
     const int tid = threadIdx.x;
     const int n = io.n;
     const int np = sm.f[0].np;
@@ -325,8 +326,8 @@ __device__ void run_tick_2f(const svpf_config_t& cfg, const SVPFParams& prm, svp
             grad_pass_2f(sm, cur, pl, cfg, prm, beta, (last && team.rank == 0) ? io.lw : nullptr);
             __syncthreads();
             if constexpr (FAST) {
-                fast_transport_2f(sm.f[0], io.v, *fw, pl.fac[0], cfg, beta, nz, kn, *fsh);
-                fast_transport_2f(sm.f[1], io.v + n, *fw, pl.fac[1], cfg, beta, nz, kn + 1, *fsh);
+                fast_transport_2f(sm.f[0], io.v, *fw, pl.fac[0], cfg, beta, nz, kn);
+                fast_transport_2f(sm.f[1], io.v + n, *fw, pl.fac[1], cfg, beta, nz, kn + 1);
             } else {
                 if (NT == kThreads || tid < kThreads) {   // a larger CTA sweeps with its first threads
                     transport_pass<R, S, 0, false, kTransport>(sm.f[0], cur, pl.fac[0], cfg, beta, nz, kn, team);
