@@ -45,6 +45,7 @@ struct svpf_stream {
     size_t smem1 = 0, smem2 = 0, smem2c = 0;
     int grid1 = 0, grid2 = 0, grid2c = 0;
     int grid1w = 0, grid2w = 0;   // of wide CTAs (WideChoice)
+    bool sweeps2 = false;   // a two-factor filter of n_max particles can sweep over its pairs on one CTA
     long long launches = 0;
     // device
     float* pool = nullptr;        // 4 arrays of pool_floats: h, h_prev, v, log_w
@@ -236,20 +237,21 @@ svpf_stream_t* svpf_stream_create(int max_instruments, size_t hbm_budget_bytes, 
         svpf_config_t any;   // the default configuration takes the fast sums
         svpf_config_init(&any, 1, SVPF_DEFAULT_NU);
         s->smem1 = tick_smem_bytes_batch(n_max, any, false);
-        s->smem2 = tick_smem_bytes_2f(n_max, 1);
         if (s->smem1 <= max_dyn_smem()) {
             s->grid1 = batch_grid(s->smem1);
             s->grid1w = batch_grid(s->smem1, true);
         }
-        if (s->smem2 <= max_dyn_smem()) {
-            const size_t fast = tick_smem_bytes_2f_fast(n_max);
-            if (fast <= max_dyn_smem()) s->smem2 = std::max(s->smem2, fast);
-            s->grid2 = batch_grid_2f(s->smem2);
-            s->grid2w = batch_grid_2f(s->smem2, true);
-        }
+        // The fast sums' layout goes further than the sweeps', which end at 5760
+        // particles: an instrument whose own fast layout fits runs on one CTA in
+        // a loop of any n_max, the others on a cluster.
+        const size_t sweeps2 = tick_smem_bytes_2f(n_max, 1);
+        s->sweeps2 = sweeps2 <= max_dyn_smem();
+        s->smem2 = std::min(std::max(s->sweeps2 ? sweeps2 : 0, tick_smem_bytes_2f_fast(n_max)), max_dyn_smem());
+        s->grid2 = batch_grid_2f(s->smem2);
+        s->grid2w = batch_grid_2f(s->smem2, true);
         s->smem2c = tick_smem_bytes_2f(n_max, kClusterMembers2f);
         if (n_max >= kClusterMinN && s->smem2c <= max_dyn_smem()) s->grid2c = batch_cluster_grid_2f(s->smem2c);
-        ok = s->grid1 > 0 || s->grid2 > 0;
+        ok = s->grid1 > 0 || (s->sweeps2 && s->grid2 > 0);
     }
     if (!ok) {
         svpf_stream_destroy(s);
@@ -289,7 +291,8 @@ int svpf_stream_admit(svpf_stream_t* s, int n, const svpf_config_t* cfg, const S
     if (!s || !cfg || !p || n < 1 || n > s->n_max) return -SVPF_ERR_INVALID_ARG;
     if (cfg->use_heun) return -SVPF_ERR_UNSUPPORTED;   // the loop's shared-memory layout has no Heun buffers
     if (!cfg->use_two_factor && s->grid1 < 1) return -SVPF_ERR_UNSUPPORTED;
-    if (cfg->use_two_factor && s->grid2 < 1 && !(n >= kClusterMinN && s->grid2c > 0)) return -SVPF_ERR_UNSUPPORTED;
+    if (cfg->use_two_factor && !(s->sweeps2 && s->grid2 > 0) && !(n >= kClusterMinN && s->grid2c > 0))
+        return -SVPF_ERR_UNSUPPORTED;
     if (cfg->use_two_factor && cfg->n_stein_steps < 1) return -SVPF_ERR_INVALID_ARG;
     if (!config_loops_ok(*cfg)) return -SVPF_ERR_INVALID_ARG;
     int slot = -1;
@@ -462,6 +465,8 @@ int svpf_stream_process_device(svpf_stream_t* s, int count1, int count2, const i
     if (!s || count1 < 0 || count2 < 0 || count1 + count2 > s->cap || !d_slots || !d_y || !d_out)
         return SVPF_ERR_INVALID_ARG;
     if (count1 + count2 == 0) return SVPF_OK;
+    // the slots are not known here: all two-factor ones must fit one CTA
+    if (count2 > 0 && !s->sweeps2) return SVPF_ERR_CUDA;
     return launch_round(s, count1, count2, d_slots, d_y, d_out);
 }
 

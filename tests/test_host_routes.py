@@ -11,3 +11,37 @@ cfg.update(use_heun=1)
 assert created(lambda: pkg.Batch([7076], [cfg], [pkg.Params(0.95, 0.1, -1.0, 0.0)]))
 assert not created(lambda: pkg.Batch([7077], [cfg], [pkg.Params(0.95, 0.1, -1.0, 0.0)]))
 """)
+
+
+def test_two_factor_instruments_take_the_fast_sums_in_a_loop_of_any_size(on_fake):  # noqa: F811
+    """An instrument of 2048 particles runs on one CTA through the fast sums
+    whatever n_max the loop was made for; one whose fast layout does not fit
+    takes a cluster.  What a loop refuses stays refused."""
+    on_fake(r"""
+cfg = pkg.default_config(2, 6.0)
+cfg.update(use_two_factor=1, rho_fast=0.8, sigma_fast=0.3, rho_slow=0.97, sigma_slow=0.1)
+prm = pkg.Params(0.95, 0.1, -3.0, 0.0)
+
+def kernels(s, slots):
+    launches()
+    s.process(np.array(slots, np.int32), np.full(len(slots), 0.3, np.float32))
+    return [(("cluster" in name), block, smem) for name, _, block, smem in launches() if "batch_tick_2f" in name]
+
+for n_max in (2048, 4096, 5760, 5761, 6000, 6464, 6465, 6784):
+    s = pkg.Stream(4, 64 << 20, n_max, seed=1)
+    a = s.admit(2048, cfg, prm)
+    ran = kernels(s, [a])
+    assert len(ran) == 1 and not ran[0][0], (n_max, ran)
+    if n_max > 5760:
+        b = s.admit(n_max, cfg, prm)
+        ran = kernels(s, [a, b])
+        assert sorted(k for k, _, _ in ran) == ([False, True] if n_max > 6464 else [False]), (n_max, ran)
+        assert s.admit(1023, cfg, prm) < 0
+        d = np.zeros(64, np.float32)
+        try:
+            s.process_device(0, 1, d.ctypes.data, d.ctypes.data, d.ctypes.data)
+            raise SystemExit("launched")
+        except RuntimeError:
+            pass
+    s.close()
+""")
