@@ -696,6 +696,9 @@ svpf_batch_t* svpf_ms_batch_inner(svpf_ms_batch_t* b);
  * predict noise, the predictive log-likelihood before the transport, and the
  * particle path cut every truncate_every ticks (0: never).  The engine has no
  * reference C counterpart; it replaces the torch model's forward/backward.
+ * Two ways to the backward, same bits: from a record of every tick, up to 4 GiB
+ * of device memory (beyond 64 MiB at most a sixteenth of what is free), or, where
+ * the records do not fit, from checkpoints every checkpoint_every ticks.
  * stream NULL: the engine makes its own stream; cudaStreamLegacy names the
  * legacy default stream. */
 typedef struct svpf_estimator svpf_estimator_t;

@@ -658,7 +658,11 @@ struct svpf_estimator {
 
 namespace {
 
-constexpr size_t kRunBytes = (size_t)4 << 30;
+// Run records hold at most kRunBytes, and beyond kRunFreely no more than a
+// kRunShare-th of the device's free memory (asking the driver for that costs
+// more than a small run).
+constexpr size_t kRunBytes = (size_t)4 << 30, kRunFreely = (size_t)64 << 20;
+constexpr size_t kRunShare = 16;
 
 template <class T>
 bool ealloc(T** p, size_t count) {
@@ -708,6 +712,56 @@ Backward backward_kernel(const svpf_estimator* e) {
     return e->d_run ? est_backward_kernel<1, true> : est_backward_kernel<1, false>;
 }
 
+// Shared memory and grid of the engine's kernels, with or without records.
+bool configure(svpf_estimator* e) {
+    // the opt-in is the device's whole limit (engines of different sizes share the kernels)
+    const void* kernels[] = {(const void*)forward_kernel(e), (const void*)backward_kernel(e)};
+    for (const void* k : kernels) {
+        if (configure_kernel(k, (int)kernel_smem_cap(k), false) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+    }
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    e->smem = (size_t)smem_floats_est(e->np, e->S, e->d_run != nullptr) * sizeof(float);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernels[1], e->threads, e->smem);
+    e->grid = std::min(e->F, std::max(1, per_sm) * std::max(sms, 1));
+    return true;
+}
+
+// Back to checkpoints, whose buffers every engine has.
+bool drop_records(svpf_estimator* e) {
+    cudaGetLastError();
+    if (!e->d_run || cudaStreamSynchronize(e->stream) != cudaSuccess) return false;
+    cudaFree(e->d_run);
+    e->d_run = nullptr;
+    e->forward_done = false;
+    return configure(e);
+}
+
+// Run records, when two of them fit in shared memory and all of them the
+// memory that is left.
+bool take_records(svpf_estimator* e, size_t optin) {
+    const size_t two = (size_t)smem_floats_est(e->np, e->S, true) * sizeof(float);
+    const size_t bytes = (size_t)e->F * e->T_max * record_floats(e->np, e->S) * sizeof(float);
+    if (two + sizeof(TickShared) + 64 > optin || bytes > kRunBytes) return true;
+    if (bytes > kRunFreely) {
+        size_t left = 0, total = 0;
+        if (cudaMemGetInfo(&left, &total) != cudaSuccess || bytes > left / kRunShare) {
+            cudaGetLastError();
+            return true;
+        }
+    }
+    if (!ealloc(&e->d_run, bytes / sizeof(float))) {
+        e->d_run = nullptr;
+        cudaGetLastError();
+        return true;
+    }
+    return configure(e) || drop_records(e);
+}
+
 }  // namespace
 
 extern "C" {
@@ -734,52 +788,33 @@ svpf_estimator_t* svpf_estimator_create(int n_filters, int n_particles, int n_st
     e->k = checkpoint_every;
     e->nseg = (T_max + checkpoint_every - 1) / checkpoint_every;
     e->trunc = truncate_every;
-    e->smem = (size_t)smem_floats_est(e->np, e->S, false) * sizeof(float);
-    int dev = 0, optin = 0, sms = 0;
+    int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e->smem + sizeof(TickShared) + 64 > (size_t)optin) {
+    if ((size_t)smem_floats_est(e->np, e->S, false) * sizeof(float) + sizeof(TickShared) + 64 > (size_t)optin) {
         delete e;
         return nullptr;
     }
     e->threads = std::min(kThreads, round_up(n_particles, 32));
-    // Run records when they take at most kRunBytes and two of them fit in
-    // shared memory.  (Asking the driver for the free memory would cost more
-    // than a small run.)
-    {
-        const size_t two = (size_t)smem_floats_est(e->np, e->S, true) * sizeof(float);
-        const size_t bytes = (size_t)n_filters * T_max * record_floats(e->np, e->S) * sizeof(float);
-        if (two + sizeof(TickShared) + 64 <= (size_t)optin && bytes <= kRunBytes &&
-            ealloc(&e->d_run, bytes / sizeof(float)))
-            e->smem = two;
-        cudaGetLastError();
-    }
     if (stream) {
         e->stream = stream;
     } else {
         cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking);
         e->own_stream = true;
     }
-    // the opt-in is the device's whole limit (engines of different sizes share the kernels)
-    const void* kernels[] = {(const void*)forward_kernel(e), (const void*)backward_kernel(e)};
-    for (const void* k : kernels) {
-        if (configure_kernel(k, (int)kernel_smem_cap(k), false) != cudaSuccess) {
-            cudaGetLastError();
-            svpf_estimator_destroy(e);
-            return nullptr;
-        }
+    if (!configure(e)) {
+        svpf_estimator_destroy(e);
+        return nullptr;
     }
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernels[1], e->threads, e->smem);
-    e->grid = std::min(n_filters, std::max(1, per_sm) * std::max(sms, 1));
     const size_t F = (size_t)n_filters, np = (size_t)e->np;
     const bool ok = ealloc(&e->d_theta, 4 * F) && ealloc(&e->d_y, F * T_max) && ealloc(&e->d_w, F * T_max) &&
                     ealloc(&e->d_loglik, F * T_max) && ealloc(&e->d_vol, F * T_max) && ealloc(&e->d_fx, F * np) &&
                     ealloc(&e->d_ck, F * e->nseg * np) && ealloc(&e->d_ax, F * np) &&
                     ealloc(&e->d_seg, (size_t)e->grid * e->k * np) && ealloc(&e->d_llsum, F) &&
                     ealloc(&e->d_ath, 4 * F) && ealloc(&e->d_status, F);
-    if (!ok) {
+    // the records last: what the checkpoints need is there without them
+    if (!ok || !take_records(e, (size_t)optin)) {
+        cudaGetLastError();
         svpf_estimator_destroy(e);
         return nullptr;
     }
@@ -852,7 +887,11 @@ int svpf_estimator_forward(svpf_estimator_t* e, const float* theta, const float*
         if (cudaStreamSynchronize(e->stream) != cudaSuccess) return SVPF_ERR_CUDA;
         cudaFree(e->d_tape);
         e->d_tape = nullptr;
-        if (!ealloc(&e->d_tape, tf)) return SVPF_ERR_CUDA;
+        if (!ealloc(&e->d_tape, tf) && !(drop_records(e) && ealloc(&e->d_tape, tf))) {
+            e->d_tape = nullptr;
+            cudaGetLastError();
+            return SVPF_ERR_CUDA;
+        }
         if (cudaMemcpyAsync(e->d_tape, tape, tf * sizeof(float), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
             return SVPF_ERR_CUDA;
         d_tape = e->d_tape;

@@ -45,3 +45,43 @@ for n_max in (2048, 4096, 5760, 5761, 6000, 6464, 6465, 6784):
             pass
     s.close()
 """)
+
+
+def test_estimator_leaves_its_records_to_what_else_needs_the_memory(on_fake):  # noqa: F811
+    """A record of every tick speeds the backward up; an engine that fits
+    without it is created, and takes a noise tape, where the memory for it is
+    short, and never takes most of what is free."""
+    on_fake(r"""
+F, T, n = 256, 100, 64
+records = F * T * (6 * 64 + 4) * 4          # 39.7 MB
+theta = np.tile(np.array([-1.0, 0.95, 0.2, 8.0], np.float32), (F, 1))
+y = np.full((F, T), 0.3, np.float32)
+
+def way(e, tape=None):
+    launches()
+    e.forward(theta, y, tape=tape)
+    e.backward()
+    return "records" if len(launches()) == 2 else "checkpoints"
+
+e = pkg.Estimator(F, n, T_max=T)
+assert way(e) == "records"
+used = fake.fake_memory_used()
+e.close()
+for spare in (0, 1 << 16, 1 << 20, 4 << 20):            # room for the records, and for part of the rest
+    fake.fake_set_memory(records + spare)
+    e = pkg.Estimator(F, n, T_max=T)
+    assert way(e) == "checkpoints", spare
+    e.close()
+fake.fake_set_memory(used)                   # no room for a tape of 3.4 MB beside them
+e = pkg.Estimator(F, n, T_max=T)
+assert way(e) == "records"
+assert way(e, np.zeros((F, e.tape_floats(n, T)), np.float32)) == "checkpoints"
+e.close()
+assert fake.fake_memory_used() == 0
+for room, want in ((64 << 30, "records"), (1 << 30, "checkpoints")):   # 159 MB of records
+    fake.fake_set_memory(room)
+    e = pkg.Estimator(4 * F, n, T_max=T)
+    theta, y = np.tile(theta[:1], (4 * F, 1)), np.full((4 * F, T), 0.3, np.float32)
+    assert way(e) == want, room
+    e.close()
+""")
