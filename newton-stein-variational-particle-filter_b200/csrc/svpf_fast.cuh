@@ -12,8 +12,10 @@
 //
 // Interpolation is by degree kP - 1 polynomials in the Chebyshev basis.  The
 // IMQ kernel 1 / (1 + u^2) has its poles at u = +-i: on a panel of half-width
-// 0.375 its expansion falls by 5.5 per degree, so kP = 12 leaves 1e-8 of the
-// sum's size (double poles included), below FP32 rounding.  The points are
+// 0.375 its expansion falls by 5.5 per degree.  With kP = 12 the largest error
+// of an interpolated kernel value is 2.5e-9 for K, 1.4e-8 for u K^2, 5.9e-8 for
+// K (3 - 4K) (the Hessian's) and 2.0e-7 for K^2 (3 - 4K) (the KSD's, three
+// poles at each end), on values of up to 1.  The points are
 // near-Chebyshev offsets rounded to 2^-14 bandwidths, so that point positions
 // and their differences are exact in FP32 and the basis change matrix
 // (inverted in rational arithmetic for those very offsets) belongs to them:
