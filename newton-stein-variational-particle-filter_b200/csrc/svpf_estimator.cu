@@ -604,6 +604,7 @@ __global__ void __launch_bounds__(kThreads, RP == 1 ? 2 : 4)
                 for (int i = tid; i < n; i += nt) s.xin[i] = sx[i];
                 __syncthreads();
                 fwd_tick<RP>(a, f, t, s, sh, s.rec, nullptr);
+                __syncthreads();   // thread 0 wrote mx, se and b last
                 const float wt = a.w ? a.w[(size_t)f * a.T + t] : 1.0f;
                 bwd_tick<RP>(smem, s.xin, sh, n, np, a.S, a.lr, a.y[(size_t)f * a.T + t], wt,
                              a.trunc > 0 && t > 0 && t % a.trunc == 0);
