@@ -432,9 +432,9 @@ int svpf_batch_tile_of(const svpf_batch_t* b, int n, int* rows_per_thread, int* 
  * (1,2) (1,1) (2,1) (4,1); SVPF_ERR_INVALID_ARG otherwise.  Forcing a tile
  * waits for the batch's stream and drops its captured graph.  A filter large
  * enough for the fast sums (more than 256 particles; two-factor, or vanilla or
- * full-Newton transport, Gaussian state noise and no Heun step) sweeps over its pairs with a
- * tile only when the tile is forced, or when its particles do not fit the
- * sums' tables. */
+ * full-Newton transport, Gaussian state noise and no Heun step) sweeps over its
+ * pairs with this tile only when it is forced: a tick whose particles do not fit
+ * the sums' tables has tiles of its own. */
 int svpf_batch_tile_of_filter(const svpf_batch_t* b, int filter, int* rows_per_thread, int* col_split);
 int svpf_batch_set_tile(svpf_batch_t* b, int filter, int rows_per_thread, int col_split);
 

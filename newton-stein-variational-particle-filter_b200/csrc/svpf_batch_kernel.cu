@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(NT, 2 * kThreads / NT) batch_tick_kernel(const
             const float ypr = readable_y_prev(yp);
             const int tile = a.tile[f];
             if (tile & kTileFast) {
-                run_tick<2, 1, false, PROD, 0, true, NT>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out);
+                run_tick<1, 1, false, PROD, 0, true, NT>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out);
             } else if constexpr (NT == kThreads) {
                 switch (tile) {
                     case 1: run_tick<1, 4, false, PROD>(cfg, prm, ctl, yt, ypr, io, nz, sm, pl, team, out); break;

@@ -560,7 +560,9 @@ __device__ __forceinline__ void push_rows(float* a, float* b, const float (&va)[
     }
 }
 
-template <int R, int S, bool STUDENT, bool SCAN = false, int U = 0>
+// NT: threads of the CTA.  More than kThreads take rows only where there are
+// more rows than the first kThreads hold.
+template <int R, int S, bool STUDENT, bool SCAN = false, int U = 0, int NT = kThreads>
 __device__ void grad_pass(const Smem& sm, int cur, const Plan& pl, const svpf_config_t& cfg,
                           float beta, float* __restrict__ lw_out, const Team& team) {
     // Positions arrive in transport coordinates hs = (h - center) / bw.  The
@@ -568,11 +570,11 @@ __device__ void grad_pass(const Smem& sm, int cur, const Plan& pl, const svpf_co
     // with sc^2 = log2(e) / (2 sigma^2), where the log-responsibility in base 2
     // is -(x - m)^2 and the sorted means m are stored scaled the same way; the
     // pair then costs one FADD, one FFMA, one ex2 and two accumulations.
-    constexpr int G = kThreads / S;
     const int grp = threadIdx.x / S, q = threadIdx.x % S;
     const float* __restrict__ hc = sm.h[cur];
     const float* __restrict__ mu = sm.mu;
     const int nloc = sm.row1 - sm.row0;
+    const int G = NT > kThreads && nloc <= R * (kThreads / S) ? kThreads / S : NT / S;
     const int nv = round_up(sm.n, 4 * S);
     const float s2 = pl.sz_eff * pl.sz_eff;
     const float inv_s2 = 1.0f / s2;
@@ -582,7 +584,7 @@ __device__ void grad_pass(const Smem& sm, int cur, const Plan& pl, const svpf_co
     const float nus2 = cfg.nu_state * s2, inv_nus2 = 1.0f / nus2, np1 = cfg.nu_state + 1.0f;
     const float half_np1 = 0.5f * np1;
 
-    for (int base = 0; base < nloc; base += G * R) {
+    for (int base = NT == kThreads || grp < G ? 0 : nloc; base < nloc; base += G * R) {
         float hj[R], xj[R], lm[R], sr[R], wg[R], wh[R];
         int jl[R];
 #pragma unroll
@@ -755,13 +757,15 @@ enum { kTransport = 0, kPhiOnly = 1, kKsdOnly = 2 };
 // (h - center) / bw) or FactorPlan (one factor of the two-factor tick:
 // positions stored in log-volatility units, scaled inside the pair FMA as
 // u = h_i / bw - h_j / bw, so the stiff per-factor priors read exact positions).
-template <int R, int S, int KIND, bool KSD, int MODE = kTransport, class P = Plan, int U = 0>
+// NT as in grad_pass.  ROWS: the rows' KSD terms go to ksd_row, by particle, and
+// nothing is returned.
+template <int R, int S, int KIND, bool KSD, int MODE = kTransport, class P = Plan, int U = 0, int NT = kThreads,
+          bool ROWS = false>
 __device__ float transport_pass(const Smem& sm, int cur, const P& pl, const svpf_config_t& cfg,
                                 float bf, const Noise& nz, int kn, const Team& team,
                                 float* __restrict__ phi_out = nullptr,
-                                const float* __restrict__ pre = nullptr) {
+                                const float* __restrict__ pre = nullptr, float* __restrict__ ksd_row = nullptr) {
     constexpr bool RAW = std::is_same<P, FactorPlan>::value;
-    constexpr int G = kThreads / S;
     const int grp = threadIdx.x / S, q = threadIdx.x % S;
     const float* __restrict__ hc = sm.h[cur];
     float* __restrict__ hn = sm.h[cur ^ 1];
@@ -769,6 +773,7 @@ __device__ float transport_pass(const Smem& sm, int cur, const P& pl, const svpf
     const float* __restrict__ cs = sm.c;
     const int n = sm.n;
     const int nloc = sm.row1 - sm.row0;
+    const int G = NT > kThreads && nloc <= R * (kThreads / S) ? kThreads / S : NT / S;
     const int nv = round_up(n, 4 * S);
     const float inv_bw = pl.inv_bw, inv_bw2 = pl.inv_bw2;
     const float sign = cfg.stein_repulsive_sign == 1 ? 1.0f : -1.0f;
@@ -777,7 +782,7 @@ __device__ float transport_pass(const Smem& sm, int cur, const P& pl, const svpf
     const float rr = cfg.rmsprop_rho;
     float ksd_thread = 0.0f;
 
-    for (int base = 0; base < nloc; base += G * R) {
+    for (int base = NT == kThreads || grp < G ? 0 : nloc; base < nloc; base += G * R) {
         float hi[R], si[R];
         float ks[R], kg[R], gk[R], kc[R], nk[R], gkr[R], gdk[R], hs[R];
         int il[R];
@@ -895,7 +900,10 @@ __device__ float transport_pass(const Smem& sm, int cur, const P& pl, const svpf
                 }
                 if (KSD) {
                     const float gsum = (KIND == 1) ? gkr[r] : gk[r];
-                    ksd_thread += si[r] * kg[r] + 2.0f * inv_bw * (si[r] * gsum - gdk[r]) + 2.0f * inv_bw2 * hs[r];
+                    if constexpr (ROWS)
+                        ksd_row[i] = si[r] * kg[r] + 2.0f * inv_bw * (si[r] * gsum - gdk[r]) + 2.0f * inv_bw2 * hs[r];
+                    else
+                        ksd_thread += si[r] * kg[r] + 2.0f * inv_bw * (si[r] * gsum - gdk[r]) + 2.0f * inv_bw2 * hs[r];
                 }
                 const int li = i - sm.row0;
                 if (MODE == kPhiOnly) { phi_out[li] = phi; continue; }

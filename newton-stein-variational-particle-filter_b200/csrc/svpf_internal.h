@@ -34,8 +34,8 @@ inline bool is_production_tick(const svpf_config_t& c) {
 // 296 / 386, 320 529 / 406.  The sweeps take 256 rows in one go, so their time
 // jumps just past that.
 constexpr int kFastMinN = 257;
-// Bit of a filter's tile byte: its ticks go through the fast sums; the tile is
-// the one its sweeps use when the particles do not fit them.
+// Bit of a filter's tile byte: its ticks go through the fast sums, and the tile
+// is not used (a tick that does not fit them has its own, sweep_any).
 constexpr int kTileFast = 0x80;
 // Two-factor filters, 592 of one size, 40 Stein steps: 200 0.86 / 1.36 ms, 256
 // 1.05 / 1.47, 320 2.36 / 1.71, 512 3.45 / 2.12, 1024 13.0 / 3.26, 2048 50.9 /

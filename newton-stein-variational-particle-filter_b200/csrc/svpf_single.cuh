@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) single_fast_kernel(const __gr
         pl.log_y2 = a.log_y2;
     }
     if (!refuse_nonfinite(a.y_t, ctl, out)) {   // every member sees the same y_t
-        run_tick<1, 1, false, PROD, 0, true, kWideThreads>(cfg, prm, ctl, a.y_t, readable_y_prev(a.y_prev), io, nz, sm,
+        run_tick<1, 4, false, PROD, 0, true, kWideThreads>(cfg, prm, ctl, a.y_t, readable_y_prev(a.y_prev), io, nz, sm,
                                                            pl, team, out);
         flag_y_prev(a.y_prev, ctl);
     }

@@ -359,6 +359,50 @@ __device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_con
     return true;
 }
 
+// One Stein iteration of a fast tick by sweeps over the pairs.  ksd: this thread's
+// KSD terms of the last iteration, summed in the order of block_reduce from the
+// prior means' place (nothing reads them again).
+template <int R, int S, bool PROD, int NT>
+__device__ __forceinline__ void sweep_iteration(const Smem& sm, int cur, const Plan& pl, const svpf_config_t& cfg,
+                                                const FilterIO& io, const Noise& nz, int kn, float beta, float bf,
+                                                bool last, const Team& team, float& ksd) {
+    grad_pass<R, S, false, false, 0, NT>(sm, cur, pl, cfg, beta, io.lw, team);
+    team.sync();
+    auto transport = [&](auto kind) {
+        constexpr int K = decltype(kind)::value;
+        if (last) transport_pass<R, S, K, true, kTransport, Plan, 0, NT, true>(sm, cur, pl, cfg, bf, nz, kn, team,
+                                                                             nullptr, nullptr, sm.mu);
+        else transport_pass<R, S, K, false, kTransport, Plan, 0, NT>(sm, cur, pl, cfg, bf, nz, kn, team);
+    };
+    if (PROD || pl.transport == 2) transport(std::integral_constant<int, 2>());
+    else transport(std::integral_constant<int, 0>());
+    if (!last) return;
+    __syncthreads();
+    ksd = 0.0f;
+    for (int i = sm.row0 + first_lane<NT>(sm.row1 - sm.row0); i < sm.row1; i += kThreads) ksd += sm.mu[i];
+}
+
+// Its tile.  On a cluster (S > 1) the widest column split up to S that takes a
+// member's rows in one go: a tick of N = 2048 315 us where one row per thread of
+// 256 took 585, 4096 976 and 1117, 8192 3.6 and 4.2 ms.  On one CTA two rows per
+// thread, on all threads of a wide one where they have rows (200 filters of 1024
+// 1.70 ms, on half of them 1.95), and four on CTAs of 256 threads above 1024
+// particles (300 of 4096 34.0 ms, two 36.8).  A wide kernel that holds a second
+// tile runs its fast iterations 0.7 % slower.  Two and four rows give the same
+// bits (the columns' order is the same; test_gpu_cta_width.py holds it), one row
+// and two did not: the compiler fuses the row's end differently.
+template <int S, bool PROD, int NT, class... A>
+__device__ __forceinline__ void sweep_any(int rows, A&&... a) {
+    if constexpr (S > 1) {
+        if (rows * S <= NT) sweep_iteration<1, S, PROD, NT>(a...);
+        else if (rows * (S / 2) <= NT) sweep_iteration<1, S / 2, PROD, NT>(a...);
+        else sweep_iteration<1, 1, PROD, NT>(a...);
+    } else {
+        if (NT == kThreads && rows > 4 * kThreads) sweep_iteration<NT == kThreads ? 4 : 2, 1, PROD, NT>(a...);
+        else sweep_iteration<2, 1, PROD, NT>(a...);
+    }
+}
+
 // The tick.  cfg/prm/ctl are shared-memory copies owned by the caller; only
 // thread 0 of rank 0 mutates ctl after make_plan.  Returns on every member; the
 // caller stores ctl/out from rank 0 thread 0.  SCAN: the mixture's row
@@ -370,7 +414,8 @@ __device__ bool fast_iteration(const FastWork& w, const Plan& pl, const svpf_con
 // FAST: the Stein iterations go through the fast sums (Gaussian state
 // noise, vanilla or full-Newton transport, no Heun step, dynamic shared memory
 // of fast_smem_floats); a tick whose particles do not fit them finishes with
-// the <R, S> sweeps.  NT: threads of the CTA (no Heun step above kThreads).
+// sweeps (sweep_any: S = 1 on one CTA, else the widest column split; R is not
+// used).  NT: threads of the CTA (no Heun step above kThreads).
 template <int R, int S, bool SCAN = false, bool PROD = false, int U = 0, bool FAST = false, int NT = kThreads>
 __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_ctl_t& ctl, float y_t,
                          float y_prev, const FilterIO& io, const Noise& nz, const Smem& sm, Plan& pl,
@@ -582,13 +627,20 @@ __device__ void run_tick(const svpf_config_t& cfg, const SVPFParams& prm, svpf_c
             }
         }
     }
-    const bool sweeps = NT == kThreads || tid < kThreads;   // a larger CTA sweeps with its first threads
+    const bool sweeps = NT == kThreads || tid < kThreads;   // small filters' one-row tiles: the first threads
     for (int it = it0; it < budget; ++it) {
         const int ai = stage_of(pl, it);
         const float beta = pl.beta[ai];
         const float bf = sqrtf(beta);
         const bool last = it == budget - 1;
-        if (PROD || !cfg.use_heun) {
+        if constexpr (FAST) {
+            float kt = 0.0f;
+            sweep_any<S, PROD, NT>((n + team.size - 1) / team.size, sm, cur, pl, cfg, io, nz, kn, beta, bf, last, team,
+                                   kt);
+            if (last) ksd_publish<NT>(kt, pl, team);
+            team.sync();
+            cur ^= 1;
+        } else if (PROD || !cfg.use_heun) {
             const float* pre = (sm.pre != nullptr && it < kPreIters) ? sm.pre + it * sm.Lp : nullptr;
             float kt = 0.0f;
             if constexpr (PROD) {

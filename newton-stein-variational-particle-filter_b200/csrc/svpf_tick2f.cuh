@@ -134,6 +134,7 @@ __device__ inline Smem2 carve_2f_fast(float* base, int n, FastWork2& w) {
 // place; v: the factor's RMSProp moments in global memory.  Positions stay in
 // log-volatility units; the sums run in bandwidths from the factor's mean.  A
 // step whose particles do not fit the tables sweeps over the pairs.
+template <int NT>
 __device__ inline void fast_transport_2f(const Smem& f, float* __restrict__ v, const FastWork2& w, const FactorPlan& fp,
                                          const svpf_config_t& cfg, float beta, const Noise& nz, int kn) {
     const int tid = threadIdx.x, nt = blockDim.x, n = f.n;
@@ -158,17 +159,14 @@ __device__ inline void fast_transport_2f(const Smem& f, float* __restrict__ v, c
     fast_bin([&](int i) { return (x[i] - cen) * ib; }, n, kFineScale, w.xs, w.pidx, t, sh);
     const Panels p = fast_panels(3, t.pt, t.comp, kFineBins / kFine, kMaxPts2f, false, t, sh);
     if (sh.over) {
-        for (int i = tid; i < n; i += nt) {
-            const float xi = x[i] * ib;
-            float kg = 0.0f, gk = 0.0f;
-            for (int j = 0; j < n; ++j) {
-                const float u = j == i ? 0.0f : fmaf(x[j], -ib, xi);
-                const float K = rcp_approx(fmaf(u, u, 1.0f));
-                kg = fmaf(K, g[j], kg);
-                gk = fmaf(u, K * K, gk);
-            }
-            w.xs[i] = move(i, v[i], kg, gk);
-        }
+        // Four rows per thread (it takes more than 1120 particles), into the binned
+        // coordinates' place.  Filters of 2048 particles of which most steps
+        // come here, 200 and 400: 5.5 and 8.0 ms a tick (one row per thread, one
+        // column at a time: 9.0 and 13.9).
+        Smem m = f;
+        m.h[1] = w.xs;
+        m.v = v;
+        transport_pass<4, 1, 0, false, kTransport, FactorPlan, 0, NT>(m, 0, fp, cfg, beta, nz, kn, Team{0, 1});
         __syncthreads();
         for (int i = tid; i < n; i += nt) x[i] = w.xs[i];
         __syncthreads();
@@ -326,8 +324,8 @@ __device__ void run_tick_2f(const svpf_config_t& cfg, const SVPFParams& prm, svp
             grad_pass_2f(sm, cur, pl, cfg, prm, beta, (last && team.rank == 0) ? io.lw : nullptr);
             __syncthreads();
             if constexpr (FAST) {
-                fast_transport_2f(sm.f[0], io.v, *fw, pl.fac[0], cfg, beta, nz, kn);
-                fast_transport_2f(sm.f[1], io.v + n, *fw, pl.fac[1], cfg, beta, nz, kn + 1);
+                fast_transport_2f<NT>(sm.f[0], io.v, *fw, pl.fac[0], cfg, beta, nz, kn);
+                fast_transport_2f<NT>(sm.f[1], io.v + n, *fw, pl.fac[1], cfg, beta, nz, kn + 1);
             } else {
                 if (NT == kThreads || tid < kThreads) {   // a larger CTA sweeps with its first threads
                     transport_pass<R, S, 0, false, kTransport>(sm.f[0], cur, pl.fac[0], cfg, beta, nz, kn, team);
