@@ -159,14 +159,15 @@ __device__ inline void fast_transport_2f(const Smem& f, float* __restrict__ v, c
     fast_bin([&](int i) { return (x[i] - cen) * ib; }, n, kFineScale, w.xs, w.pidx, t, sh);
     const Panels p = fast_panels(3, t.pt, t.comp, kFineBins / kFine, kMaxPts2f, false, t, sh);
     if (sh.over) {
-        // Four rows per thread (it takes more than 1120 particles), into the binned
+        // One row per thread, in packed column pairs, into the binned
         // coordinates' place.  Filters of 2048 particles of which most steps
-        // come here, 200 and 400: 5.5 and 8.0 ms a tick (one row per thread, one
-        // column at a time: 9.0 and 13.9).
+        // come here, 200 and 400: 6.2 and 9.2 ms a tick (one column at a time: 9.0
+        // and 13.9; four rows per thread 5.6 and 8.1, but that code costs the steps
+        // that fit 1 %).
         Smem m = f;
         m.h[1] = w.xs;
         m.v = v;
-        transport_pass<4, 1, 0, false, kTransport, FactorPlan, 0, NT>(m, 0, fp, cfg, beta, nz, kn, Team{0, 1});
+        transport_pass<1, 1, 0, false, kTransport, FactorPlan, 0, NT>(m, 0, fp, cfg, beta, nz, kn, Team{0, 1});
         __syncthreads();
         for (int i = tid; i < n; i += nt) x[i] = w.xs[i];
         __syncthreads();
